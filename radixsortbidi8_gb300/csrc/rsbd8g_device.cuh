@@ -23,6 +23,10 @@ namespace rsbd8g {
 constexpr int kRadixBits = 8;
 constexpr int kBuckets = 1 << kRadixBits;
 constexpr int kMaxPasses = 16;   // 128-bit keys: 16 digit passes
+// A sort of 8- or 16-byte keys has kPrefixSlots pass launches ahead of the settle launch and one per
+// digit after it (see rsbd8g_prefix.cuh); other sorts have one per digit.
+constexpr int kPrefixSlots = 6;
+constexpr int kMaxSlots = kPrefixSlots + kMaxPasses;
 
 // device status bits (Control::error)
 enum : uint32_t { kDevTimeout = 1u, kDevFault = 2u };
@@ -73,7 +77,8 @@ struct PassPlan {
     uint32_t reverse;      // read the source back to front (isrevorder, first surviving pass)
     uint32_t hot;          // crowded digits of the pass, ranked with ballots: (digit1 << 16) | digit0,
                            // kNoHot in a half for none (see TileRank)
-    uint32_t pad1;
+    uint16_t digit;        // the digit this launch sorts by
+    uint16_t status;       // its array of look-back words
 };
 constexpr uint32_t kNoHot = 0x100u;                       // not a digit: matches no key
 constexpr uint32_t kNoHotPair = (kNoHot << 16) | kNoHot;
@@ -81,7 +86,7 @@ constexpr uint32_t kNoHotPair = (kNoHot << 16) | kNoHot;
 struct Control {
     uint32_t error;
     uint32_t abort;
-    uint32_t tile_counter[kMaxPasses];
+    uint32_t tile_counter[kMaxSlots];
     uint32_t active_passes;
     uint32_t copy_mode;
     uint32_t copy_src;     // SortArrays indices
@@ -89,9 +94,16 @@ struct Control {
     uint32_t stall_tile;   // diagnostics: this tile never publishes (0xFFFFFFFF = off)
     uint32_t prefetch;     // 1: every array is device memory, so tiles may be prefetched into L2
     uint32_t hist_done;    // histogram CTAs finished (the last one computes the plan)
+    uint32_t prefix_low;   // prefix sort: the lowest digit of the prefix the passes sorted by
+    uint32_t prefix_passes; // prefix sort: passes before the settle launch (0: a plain LSD sort)
+    uint32_t settle_fail;  // a group of equal prefixes could not be settled: the plain passes run
+    uint32_t settle_done;  // settle CTAs finished (the last one plans the plain passes if they are needed)
+    uint32_t survive;      // digits that are not all in one bucket (bit per digit)
+    uint32_t sample_pairs[kMaxPasses];   // sample key pairs by their highest differing digit
+    uint32_t hot[kMaxPasses];            // crowded digits of each digit position (PassPlan::hot)
     uint32_t pad0;
     uint64_t spin_limit_ns;
-    PassPlan plan[kMaxPasses];
+    PassPlan plan[kMaxSlots];
 };
 static_assert(sizeof(Control) <= 1024, "control block must fit its slot");
 
@@ -208,6 +220,36 @@ __host__ __device__ __forceinline__ KeyWide<HB> filter_key(KeyWide<HB> b) {
         if constexpr (SIGN) return K{lo, hi ^ sb};                           // signed, MSB flip
         return K{lo, hi};                                                    // unsigned
     }
+}
+
+// order, equality and digit comparisons of filtered keys
+template <typename U>
+__host__ __device__ __forceinline__ bool key_less(U a, U b) { return a < b; }
+template <int HB>
+__host__ __device__ __forceinline__ bool key_less(KeyWide<HB> a, KeyWide<HB> b) {
+    return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo);
+}
+template <typename U>
+__host__ __device__ __forceinline__ bool key_same(U a, U b) { return a == b; }
+template <int HB>
+__host__ __device__ __forceinline__ bool key_same(KeyWide<HB> a, KeyWide<HB> b) { return a.hi == b.hi && a.lo == b.lo; }
+// the bits of every digit from `low` up, and keys that are equal in the bits of m
+template <typename U>
+__device__ __forceinline__ U prefix_mask(uint32_t low) {
+    if constexpr (sizeof(U) == 8) return ~U(0) << (low * kRadixBits);
+    else return U{low < 8 ? ~uint64_t(0) << (low * kRadixBits) : 0u, low < 8 ? ~uint64_t(0) : ~uint64_t(0) << ((low - 8) * kRadixBits)};
+}
+template <typename U>
+__device__ __forceinline__ bool same_masked(U a, U b, U m) { return ((a ^ b) & m) == 0; }
+template <int HB>
+__device__ __forceinline__ bool same_masked(KeyWide<HB> a, KeyWide<HB> b, KeyWide<HB> m) {
+    return (((a.lo ^ b.lo) & m.lo) | ((a.hi ^ b.hi) & m.hi)) == 0;
+}
+// the highest digit in which a and b differ (a != b)
+__device__ __forceinline__ uint32_t top_diff(uint64_t a, uint64_t b) { return (63u - uint32_t(__clzll(a ^ b))) / kRadixBits; }
+template <int HB>
+__device__ __forceinline__ uint32_t top_diff(KeyWide<HB> a, KeyWide<HB> b) {
+    return a.hi != b.hi ? 8u + top_diff(a.hi, b.hi) : top_diff(a.lo, b.lo);
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {

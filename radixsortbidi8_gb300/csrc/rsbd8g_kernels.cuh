@@ -22,22 +22,11 @@
 //                                      when every pass was skipped, and the last pass's launch does it)
 #pragma once
 #include "rsbd8g_device.cuh"
+#include "rsbd8g_prefix.cuh"
 
 namespace rsbd8g {
 
 // ---- scan, pass-skip and plan -----------------------------------------------------------------
-
-struct PlanArgs {
-    uint64_t spin_limit_ns;
-    uint32_t inplace;      // radixsort / radixsortnoalloc: sort `in` using `buf`
-    uint32_t to_buffer;    // movetobuffer
-    uint32_t rev;          // effective isrevorder
-    uint32_t indirect;
-    uint32_t stall_tile;
-    uint32_t passes;       // digits of the key
-    uint32_t prefetch;     // every array is device memory (Control::prefetch)
-    uint32_t hot_ok;       // crowded digits may be ranked with ballots (PassPlan::hot)
-};
 
 // a digit is ranked with ballots (PassPlan::hot) when it holds more than 1/kHotShare of the keys: the
 // ballots cost every key of the pass instructions (about 30 % more time on a pass of uniform digits
@@ -79,9 +68,11 @@ __device__ __forceinline__ unsigned long long plan_block_max(unsigned long long 
 __device__ __forceinline__ void plan_body(Control *__restrict__ ctrl, const unsigned long long *__restrict__ ghist,
                                           unsigned long long *__restrict__ bstart, uint64_t n, const PlanArgs &a) {
     __shared__ unsigned long long wsum[kBuckets / 32];
-    __shared__ int skip[kMaxPasses];
-    __shared__ uint32_t hot[kMaxPasses];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    __shared__ uint32_t hot[kMaxPasses], pairs[kMaxPasses];    // (thread 0 plans from shared memory: a chain of
+                                                               // loads from L2 would take 10 us)
+    if (a.prefix_ok && t < kMaxPasses) pairs[t] = __ldcg(&ctrl->sample_pairs[t]);
+    uint32_t survive = 0;
     for (int p = 0; p < int(a.passes); ++p) {
         // the other CTAs' counts arrive through L2 (their atomics were fenced before they finished)
         const unsigned long long h = __ldcg(ghist + p * kBuckets + t);
@@ -92,7 +83,9 @@ __device__ __forceinline__ void plan_body(Control *__restrict__ ctrl, const unsi
         if (t == 0) {
             const uint32_t h0 = (m0 >> 8) > n / kHotShare ? uint32_t(m0 & 0xFFu) : kNoHot;
             hot[p] = a.hot_ok ? ((kNoHot << 16) | h0) : kNoHotPair;
+            if (a.prefix_ok) ctrl->hot[p] = hot[p];
         }
+        if (!all_in_one) survive |= 1u << p;
         unsigned long long x = h;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -104,62 +97,26 @@ __device__ __forceinline__ void plan_body(Control *__restrict__ ctrl, const unsi
         unsigned long long before = 0;
         for (int i = 0; i < w; ++i) before += wsum[i];
         bstart[p * kBuckets + t] = before + x - h;
-        if (t == 0) skip[p] = all_in_one;
         plan_sync();
     }
     if (t != 0) return;
-    int k = 0;
-    for (int p = 0; p < int(a.passes); ++p) k += !skip[p];
-    ctrl->active_passes = uint32_t(k);
+    ctrl->active_passes = uint32_t(__popc(survive));
+    ctrl->survive = survive;
     ctrl->spin_limit_ns = a.spin_limit_ns;
     ctrl->stall_tile = a.stall_tile;
     ctrl->prefetch = a.prefetch;
-    ctrl->copy_mode = kCopyNone;
-    uint32_t cur = kArrIn;                // where the data (values for indirection) is
-    uint32_t curk = kArrKeysA;            // indirection: where the filtered keys are
-    int i = 0;
-    for (int p = 0; p < int(a.passes); ++p) {
-        PassPlan &pp = ctrl->plan[p];
-        pp.active = !skip[p];
-        pp.hot = hot[p];
-        if (skip[p]) continue;
-        ++i;
-        uint32_t dst;
-        if (a.inplace) dst = (cur == kArrIn) ? kArrBuf : kArrIn;
-        else dst = ((k - i) % 2 == 0) ? kArrOut : kArrBuf;
-        pp.reverse = (i == 1) && a.rev;
-        if (a.indirect) {
-            pp.src_vals = cur;
-            pp.dst_vals = dst;
-            pp.src_keys = curk;
-            const uint32_t dk = (curk == kArrKeysA) ? kArrKeysB : kArrKeysA;
-            pp.dst_keys = (i == k) ? kArrNone : dk;
-            curk = dk;
-        } else {
-            pp.src_keys = cur;
-            pp.dst_keys = dst;
-            pp.src_vals = kArrNone;
-            pp.dst_vals = kArrNone;
-        }
-        cur = dst;
-    }
-    if (!a.inplace) {
-        if (k == 0) {
-            ctrl->copy_mode = a.rev ? kCopyReversed : kCopyPlain;
-            ctrl->copy_src = kArrIn;
-            ctrl->copy_dst = kArrOut;
-        }
+    uint32_t curk = kArrKeysA, low = 0;
+    const uint32_t k = a.prefix_ok ? prefix_choose(pairs, survive, n, uint64_t(prefix_rounds(n)) * gridDim.x * blockDim.x * (blockDim.x - 1u) / 2u,
+                                                     &low) : 0u;
+    ctrl->prefix_passes = k;
+    ctrl->prefix_low = low;
+    if (k) {
+        // the prefix passes, then the settle launch in place where they end
+        const uint32_t cur = plan_chain(ctrl, a, hot, survive & ~((1u << low) - 1u), false, 0, kArrIn, curk, a.rev != 0, true);
+        plan_copy(ctrl, a, cur, false);
     } else {
-        const uint32_t target = a.to_buffer ? kArrBuf : kArrIn;
-        if (k == 0 && a.rev) {
-            ctrl->copy_mode = a.to_buffer ? kCopyReversed : kReverseInPlace;
-            ctrl->copy_src = kArrIn;
-            ctrl->copy_dst = target;
-        } else if (cur != target) {
-            ctrl->copy_mode = kCopyPlain;
-            ctrl->copy_src = cur;
-            ctrl->copy_dst = target;
-        }
+        const uint32_t cur = plan_chain(ctrl, a, hot, survive, false, 0, kArrIn, curk, a.rev != 0, false);
+        plan_copy(ctrl, a, cur, survive == 0u);
     }
 }
 
@@ -240,6 +197,10 @@ __global__ void __launch_bounds__(THREADS) k_histogram(const U *__restrict__ key
     constexpr int C = hist_lane_copies<P>();
     constexpr int V = 16 / int(sizeof(U));
     extern __shared__ __align__(16) uint32_t shl[];
+    if constexpr (P >= 8) {
+        if (pa.prefix_ok)
+            prefix_sample<U, THREADS>(reinterpret_cast<U *>(shl), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(keys[i]); });
+    }
     for (int i = threadIdx.x; i < C * P * kBuckets; i += THREADS) shl[i] = 0;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
@@ -298,7 +259,17 @@ __global__ void __launch_bounds__(THREADS) k_gather_histogram(const uint64_t *__
                                                               Control *__restrict__ ctrl,
                                                               unsigned long long *__restrict__ bstart, PlanArgs pa) {
     constexpr int P = KeyTraits<U>::kDigits;
-    __shared__ uint32_t shall[gather_hist_copies<P>() * P * kBuckets];
+    __shared__ __align__(16) uint32_t shall[gather_hist_copies<P>() * P * kBuckets];
+    auto key_at = [&](uint64_t i) {
+        if (level == 3) return keys_in[i];
+        const unsigned char *obj = reinterpret_cast<const unsigned char *>(ptrs[i]) + off1;
+        if (level == 2) obj = load_ptr(obj) + off2;
+        return load_member<U>(obj);
+    };
+    if constexpr (P >= 8) {
+        if (pa.prefix_ok)
+            prefix_sample<U, THREADS>(reinterpret_cast<U *>(shall), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(key_at(i)); });
+    }
     zero_hist<THREADS, P>(shall);
     uint32_t *sh = shall + ((threadIdx.x >> 5) % gather_hist_copies<P>()) * P * kBuckets;
     const uint32_t lane = threadIdx.x & 31u;
@@ -311,15 +282,7 @@ __global__ void __launch_bounds__(THREADS) k_gather_histogram(const uint64_t *__
         for (int u = 0; u < UNR; ++u) {
             const uint64_t i = b + u * 32 + lane;
             raw[u] = U{};
-            if (i < n) {
-                if (level == 3) {
-                    raw[u] = keys_in[i];
-                } else {
-                    const unsigned char *obj = reinterpret_cast<const unsigned char *>(ptrs[i]) + off1;
-                    if (level == 2) obj = load_ptr(obj) + off2;
-                    raw[u] = load_member<U>(obj);
-                }
-            }
+            if (i < n) raw[u] = key_at(i);
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
@@ -848,7 +811,7 @@ template <typename U, int MODE, bool HAS_VAL, int THREADS, int ITEMS, typename S
 __device__ __forceinline__ void onesweep_body(unsigned char *smem, Control *__restrict__ ctrl,
                                               const PassPlan &plan, const SortArrays &arrs,
                                               const unsigned long long *__restrict__ bstart_all,
-                                              S *__restrict__ status, int pass, uint64_t n, uint32_t num_tiles,
+                                              S *__restrict__ status, int slot, int pass, uint64_t n, uint32_t num_tiles,
                                               uint32_t dmask) {
     using L = OnesweepSmem<U, HAS_VAL, THREADS, ITEMS>;
     unsigned long long *bstart = reinterpret_cast<unsigned long long *>(smem + L::kOffBstart);
@@ -873,7 +836,7 @@ __device__ __forceinline__ void onesweep_body(unsigned char *smem, Control *__re
     sweep_init_smem<U, MODE, HAS_VAL, THREADS, ITEMS, S>(smem);
     for (;;) {
         if (threadIdx.x == 0) {
-            const uint32_t tile = atomicAdd(&ctrl->tile_counter[pass], 1u);
+            const uint32_t tile = atomicAdd(&ctrl->tile_counter[slot], 1u);
             misc[0] = tile;
             misc[1] = 0;
             // the tile one grid stride on is about the next one any CTA claims: its data go to L2 now
@@ -896,23 +859,27 @@ __device__ __forceinline__ void onesweep_body(unsigned char *smem, Control *__re
 template <typename U, int MODE, bool HAS_VAL, int THREADS, int ITEMS, typename S>
 __global__ void __launch_bounds__(THREADS, onesweep_min_blocks<U, HAS_VAL, THREADS>())
     k_onesweep(Control *__restrict__ ctrl, const SortArrays arrs, const unsigned long long *__restrict__ bstart_all,
-               S *__restrict__ status, int pass, uint64_t n, uint32_t num_tiles, uint32_t dmask, uint32_t fold_copy) {
+               S *__restrict__ status_all, size_t status_stride, int slot, uint64_t n, uint32_t num_tiles, uint32_t dmask,
+               uint32_t fold_copy) {
     using L = OnesweepSmem<U, HAS_VAL, THREADS, ITEMS>;
     static_assert(THREADS >= kBuckets && THREADS % 32 == 0, "one thread per digit");
     static_assert(L::kTile <= 65535, "tile ranks are 16-bit");
     extern __shared__ __align__(16) unsigned char smem[];
-    const PassPlan plan = ctrl->plan[pass];
+    const PassPlan plan = ctrl->plan[slot];
     if (!plan.active) {
         // the last pass of a copy form: when every pass was skipped, the copy the plan asks for
         if (fold_copy) copy_step(ctrl, arrs, n, HAS_VAL ? 8u : uint32_t(sizeof(U)));
         return;
     }
+    // keys of up to 4 bytes sort by digit `slot` in launch `slot`; the plan of wider keys names the digit
+    const int pass = KeyTraits<U>::kDigits >= 8 ? int(plan.digit) : slot;
+    S *status = status_all + status_stride * (KeyTraits<U>::kDigits >= 8 ? uint32_t(plan.status) : 0u);
     // a crowded pass ranks its hot digits with ballots (the choice is uniform over the launch)
     if (plan.hot == kNoHotPair)
-        onesweep_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 0>(smem, ctrl, plan, arrs, bstart_all, status, pass, n, num_tiles,
+        onesweep_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 0>(smem, ctrl, plan, arrs, bstart_all, status, slot, pass, n, num_tiles,
                                                               dmask);
     else
-        onesweep_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 1>(smem, ctrl, plan, arrs, bstart_all, status, pass, n, num_tiles,
+        onesweep_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 1>(smem, ctrl, plan, arrs, bstart_all, status, slot, pass, n, num_tiles,
                                                               dmask);
 }
 
@@ -947,7 +914,7 @@ template <typename U, int MODE, bool HAS_VAL, int THREADS, int ITEMS, typename S
 __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control *__restrict__ ctrl, const PassPlan &plan,
                                                    const SortArrays &arrs,
                                                    const unsigned long long *__restrict__ bstart_all,
-                                                   S *__restrict__ status, int pass, uint64_t n, uint32_t num_tiles,
+                                                   S *__restrict__ status, int slot, int pass, uint64_t n, uint32_t num_tiles,
                                                    uint32_t dmask) {
     using L = PipeSmem<U, THREADS, ITEMS, HAS_VAL>;
     constexpr int TILE = L::kTile;
@@ -990,7 +957,7 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
     for (int i = tid; i < kBuckets; i += THREADS) bstart[i] = bstart_all[pass * kBuckets + i];
     for (int i = tid; i < R::kWords; i += THREADS) utab[i] = 0u;
     if (tid == 0) {
-        misc[0] = atomicAdd(&ctrl->tile_counter[pass], 1u);
+        misc[0] = atomicAdd(&ctrl->tile_counter[slot], 1u);
         misc[1] = 0u;
     }
     __syncthreads();
@@ -1005,7 +972,7 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
         uint32_t *cntB = cntall + par * kBuckets, *cntA = cntall + (par ^ 1) * kBuckets;
         uint32_t next = 0xFFFFFFFFu;
         if (hasB && tid == 0) {
-            next = atomicAdd(&ctrl->tile_counter[pass], 1u);   // the tile after B: its keys go to L2 now
+            next = atomicAdd(&ctrl->tile_counter[slot], 1u);   // the tile after B: its keys go to L2 now
             if (prefetch && next < num_tiles) {
                 prefetch_tile<TILE>(src, n, next, reverse);
                 if constexpr (HAS_VAL) prefetch_tile<TILE>(src_v, n, next, reverse);
@@ -1152,23 +1119,26 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
 template <typename U, int MODE, bool HAS_VAL, int THREADS, int ITEMS, typename S>
 __global__ void __launch_bounds__(THREADS, 2)
     k_onesweep_pipe(Control *__restrict__ ctrl, const SortArrays arrs, const unsigned long long *__restrict__ bstart_all,
-                    S *__restrict__ status, int pass, uint64_t n, uint32_t num_tiles, uint32_t dmask,
+                    S *__restrict__ status_all, size_t status_stride, int slot, uint64_t n, uint32_t num_tiles, uint32_t dmask,
                     uint32_t fold_copy) {
     static_assert(THREADS == 2 * kBuckets, "threads 0..255 scan, threads 256..511 look back");
     static_assert(PipeSmem<U, THREADS, ITEMS, HAS_VAL>::kTile <= 65535, "tile ranks are 16-bit");
     extern __shared__ __align__(16) unsigned char smem[];
-    const PassPlan plan = ctrl->plan[pass];
+    const PassPlan plan = ctrl->plan[slot];
     if (!plan.active) {
         // the last pass of a copy form: when every pass was skipped, the copy the plan asks for
         if (fold_copy) copy_step(ctrl, arrs, n, HAS_VAL ? 8u : uint32_t(sizeof(U)));
         return;
     }
+    // keys of up to 4 bytes sort by digit `slot` in launch `slot`; the plan of wider keys names the digit
+    const int pass = KeyTraits<U>::kDigits >= 8 ? int(plan.digit) : slot;
+    S *status = status_all + status_stride * (KeyTraits<U>::kDigits >= 8 ? uint32_t(plan.status) : 0u);
     // a crowded pass ranks its hot digits with ballots (the choice is uniform over the launch)
     if (plan.hot == kNoHotPair)
-        onesweep_pipe_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 0>(smem, ctrl, plan, arrs, bstart_all, status, pass, n,
+        onesweep_pipe_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 0>(smem, ctrl, plan, arrs, bstart_all, status, slot, pass, n,
                                                                    num_tiles, dmask);
     else
-        onesweep_pipe_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 1>(smem, ctrl, plan, arrs, bstart_all, status, pass, n,
+        onesweep_pipe_body<U, MODE, HAS_VAL, THREADS, ITEMS, S, 1>(smem, ctrl, plan, arrs, bstart_all, status, slot, pass, n,
                                                                    num_tiles, dmask);
 }
 

@@ -50,9 +50,34 @@ struct SweepKernels {
     }
 };
 
+// resident CTAs per SM of the settle kernel on device `dev` (which also loads it)
+template <typename U, int MODE, bool HAS_VAL>
+int settle_setup(int dev) {
+    static std::once_flag once[64];
+    static int occ[64];
+    std::call_once(once[dev & 63], [&] {
+        int b = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_settle<U, MODE, HAS_VAL>, SettleShape<U>::kThreads, 0);
+        occ[dev & 63] = b > 0 ? b : 1;
+    });
+    return occ[dev & 63];
+}
+
+template <typename U, int MODE, bool HAS_VAL>
+cudaError_t launch_settle_t(uint64_t n, const Layout &L, unsigned char *scratch, const SortArrays &arrs, uint32_t dmask,
+                            const PlanArgs &pa, cudaStream_t s) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t tiles = (n + SettleShape<U>::kCtaKeys - 1) / SettleShape<U>::kCtaKeys;
+    const uint64_t resident = uint64_t(settle_setup<U, MODE, HAS_VAL>(dev)) * device_sms(dev);
+    k_settle<U, MODE, HAS_VAL><<<uint32_t(std::min(tiles, resident)), SettleShape<U>::kThreads, 0, s>>>(
+        reinterpret_cast<Control *>(scratch + L.ctrl), arrs, n, dmask, scratch + L.status, L.status_pass_bytes, pa);
+    return cudaGetLastError();
+}
+
 template <typename U, int MODE, bool HAS_VAL, int THREADS, int ITEMS, typename S>
 cudaError_t launch_sweeps_t(uint32_t passes, uint64_t n, const Layout &L, unsigned char *scratch,
-                            const SortArrays &arrs, uint32_t dmask, bool fold_copy, cudaStream_t s) {
+                            const SortArrays &arrs, uint32_t dmask, bool fold_copy, const PlanArgs &pa, cudaStream_t s) {
     // the pipelined pass, unless there are too few tiles to fill its pipeline (a sort of about one
     // tile per CTA runs each tile's phases back to back in k_onesweep instead)
     using K = SweepKernels<U, MODE, HAS_VAL, THREADS, ITEMS, S>;
@@ -69,14 +94,25 @@ cudaError_t launch_sweeps_t(uint32_t passes, uint64_t n, const Layout &L, unsign
     const uint32_t grid = uint32_t(std::min<uint64_t>(L.num_tiles, pipe ? resident : uint64_t(occ) * device_sms(dev)));
     Control *ctrl = reinterpret_cast<Control *>(scratch + L.ctrl);
     const unsigned long long *bstart = reinterpret_cast<const unsigned long long *>(scratch + L.bstart);
-    for (uint32_t p = 0; p < passes; ++p) {
-        S *status = reinterpret_cast<S *>(scratch + L.status + size_t(p) * L.status_pass_bytes);
+    S *status = reinterpret_cast<S *>(scratch + L.status);
+    const size_t stride = L.status_pass_bytes / sizeof(S);
+    const uint32_t slots = passes + (pa.prefix_ok ? uint32_t(kPrefixSlots) : 0u);
+    for (uint32_t p = 0; p < slots; ++p) {
+        if constexpr (KeyTraits<U>::kDigits >= 8) {
+            if (pa.prefix_ok && p == uint32_t(kPrefixSlots)) {
+                LaunchTimer t(s, RSBD8G_KERNEL_SETTLE, uint32_t(sizeof(U)), 0, n);
+                const cudaError_t e = launch_settle_t<U, MODE, HAS_VAL>(n, L, scratch, arrs, dmask, pa, s);
+                if (e != cudaSuccess) return e;
+            }
+        }
         LaunchTimer t(s, RSBD8G_KERNEL_ONESWEEP, uint32_t(sizeof(U)), p, n);
-        const uint32_t fc = (fold_copy && p + 1 == passes) ? 1u : 0u;   // the copy forms' copy, in the last pass
+        // the look-back words of a pass: the launch's own, or as the plan of wider keys names them
+        S *st = status + (KeyTraits<U>::kDigits >= 8 ? 0 : size_t(p) * stride);
+        const uint32_t fc = (fold_copy && p + 1 == slots) ? 1u : 0u;   // the copy forms' copy, in the last pass
         if (pipe)
-            pkern<<<grid, THREADS, PM::kBytes, s>>>(ctrl, arrs, bstart, status, int(p), n, L.num_tiles, dmask, fc);
+            pkern<<<grid, THREADS, PM::kBytes, s>>>(ctrl, arrs, bstart, st, stride, int(p), n, L.num_tiles, dmask, fc);
         else
-            kern<<<grid, THREADS, SM::kBytes, s>>>(ctrl, arrs, bstart, status, int(p), n, L.num_tiles, dmask, fc);
+            kern<<<grid, THREADS, SM::kBytes, s>>>(ctrl, arrs, bstart, st, stride, int(p), n, L.num_tiles, dmask, fc);
     }
     return cudaGetLastError();
 }
@@ -112,6 +148,7 @@ cudaError_t launch_histogram_t(const Resolved &r, uint64_t n, const void *in, co
     } else {
         constexpr int P = KeyTraits<U>::kDigits;
         constexpr size_t smem = size_t(hist_lane_copies<P>()) * P * kBuckets * 4;
+        static_assert(kHistDirectThreads * sizeof(U) <= smem, "the sample fits the counters' memory");
         auto kern = k_histogram<U, MODE, kHistDirectThreads>;
         histogram_setup<U, MODE>(dev);
         const uint64_t per = uint64_t(kHistDirectThreads) * 16;   // at least 16 keys a thread
@@ -151,6 +188,7 @@ cudaError_t launch_sort_t(const Resolved &r, uint64_t n, const Layout &L, unsign
     a.prefetch = r.prefetch;
     a.hot_ok = 1u;
     const bool stall = (r.flags & RSBD8G_FLAG_DIAG_STALL) != 0;
+    a.prefix_ok = KeyTraits<U>::kDigits >= 8 && n >= prefix_min_keys(int(sizeof(U))) && !stall;
     a.stall_tile = stall ? 1u : 0xFFFFFFFFu;
     a.spin_limit_ns = stall ? 200000000ull : 1000000000ull;
     // the histograms; the CTA that finishes them last writes the plan
@@ -161,22 +199,22 @@ cudaError_t launch_sort_t(const Resolved &r, uint64_t n, const Layout &L, unsign
     const uint32_t P = uint32_t(KeyTraits<U>::kDigits);
     if (r.indirect) {
         e = L.wide_status
-                ? launch_sweeps_t<U, 0, true, gi.threads, gi.items, uint64_t>(P, n, L, scratch, arrs, 0u, !inplace, s)
-                : launch_sweeps_t<U, 0, true, gi.threads, gi.items, uint32_t>(P, n, L, scratch, arrs, 0u, !inplace, s);
+                ? launch_sweeps_t<U, 0, true, gi.threads, gi.items, uint64_t>(P, n, L, scratch, arrs, 0u, !inplace, a, s)
+                : launch_sweeps_t<U, 0, true, gi.threads, gi.items, uint32_t>(P, n, L, scratch, arrs, 0u, !inplace, a, s);
     } else if (L.wide_status) {
-#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gd.threads, gd.items, uint64_t>(P, n, L, scratch, arrs, dmask, !inplace, s)
+#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gd.threads, gd.items, uint64_t>(P, n, L, scratch, arrs, dmask, !inplace, a, s)
         RSBD8G_MODE_SWITCH(mode, RSBD8G_SWEEP)
 #undef RSBD8G_SWEEP
     } else if (L.large_tiles) {
-#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gl.threads, gl.items, uint32_t>(P, n, L, scratch, arrs, dmask, !inplace, s)
+#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gl.threads, gl.items, uint32_t>(P, n, L, scratch, arrs, dmask, !inplace, a, s)
         RSBD8G_MODE_SWITCH(mode, RSBD8G_SWEEP)
 #undef RSBD8G_SWEEP
     } else if (L.small_tiles) {
-#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gs.threads, gs.items, uint32_t>(P, n, L, scratch, arrs, dmask, !inplace, s)
+#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gs.threads, gs.items, uint32_t>(P, n, L, scratch, arrs, dmask, !inplace, a, s)
         RSBD8G_MODE_SWITCH(mode, RSBD8G_SWEEP)
 #undef RSBD8G_SWEEP
     } else {
-#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gd.threads, gd.items, uint32_t>(P, n, L, scratch, arrs, dmask, !inplace, s)
+#define RSBD8G_SWEEP(M) e = launch_sweeps_t<U, M, false, gd.threads, gd.items, uint32_t>(P, n, L, scratch, arrs, dmask, !inplace, a, s)
         RSBD8G_MODE_SWITCH(mode, RSBD8G_SWEEP)
 #undef RSBD8G_SWEEP
     }
@@ -204,12 +242,14 @@ cudaError_t prepare_mode_t(bool indirect, int dev) {
         cudaFuncGetAttributes(&fa, k_gather_histogram<U, MODE, kHistThreads>);
         SweepKernels<U, 0, true, gi.threads, gi.items, uint32_t>::setup(dev, nullptr, nullptr);
         SweepKernels<U, 0, true, gi.threads, gi.items, uint64_t>::setup(dev, nullptr, nullptr);
+        if constexpr (KeyTraits<U>::kDigits >= 8) settle_setup<U, 0, true>(dev);
     } else {
         histogram_setup<U, MODE>(dev);
         SweepKernels<U, MODE, false, gd.threads, gd.items, uint32_t>::setup(dev, nullptr, nullptr);
         SweepKernels<U, MODE, false, gd.threads, gd.items, uint64_t>::setup(dev, nullptr, nullptr);
         SweepKernels<U, MODE, false, gl.threads, gl.items, uint32_t>::setup(dev, nullptr, nullptr);
         SweepKernels<U, MODE, false, gs.threads, gs.items, uint32_t>::setup(dev, nullptr, nullptr);
+        if constexpr (KeyTraits<U>::kDigits >= 8) settle_setup<U, MODE, false>(dev);
     }
     cudaFuncGetAttributes(&fa, k_copy);
     return cudaGetLastError();

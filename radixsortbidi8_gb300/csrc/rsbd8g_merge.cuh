@@ -22,13 +22,6 @@ __host__ __device__ __forceinline__ U order_key(U b, bool desc) {
     return desc ? key_not(k) : k;
 }
 
-template <typename U>
-__host__ __device__ __forceinline__ bool key_less(U a, U b) { return a < b; }
-template <int HB>
-__host__ __device__ __forceinline__ bool key_less(KeyWide<HB> a, KeyWide<HB> b) {
-    return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo);
-}
-
 // does a (from run A) go before b (from run B)?  a_first: A has precedence on equal keys
 template <int MODE, typename U>
 __host__ __device__ __forceinline__ bool a_before_b(U a, U b, bool desc, bool a_first) {

@@ -1,0 +1,492 @@
+// rsbd8g_prefix.cuh - the prefix sort of 8- and 16-byte keys.
+//
+// An LSD sort of n keys runs one scatter pass per digit, but where the keys are spread out the top
+// few digits already tell nearly all of them apart: 2^28 uniform 64-bit keys share their top 32 bits
+// with one other key in 16.  So a large sort of wide keys first runs stable passes over a prefix --
+// the top digits that are not all in one bucket -- and then settles the short groups of keys whose
+// prefixes are equal, in one read of the keys:
+//   * prefix_sample   each CTA of the histogram launch sorts a small random sample of the keys and
+//                     counts, by highest differing digit, the neighbours that differ
+//   * prefix_choose   (in the plan) the shortest prefix whose sample pairs leave groups of few keys on
+//                     average; none when the sample says that more than kPrefixSlots digits, or nearly
+//                     all of them, are needed: then the plain LSD passes run
+//   * k_settle        puts every group of equal prefixes into the order of the whole keys, ties in
+//                     the order they came (the passes were stable), so the result is the LSD sort's
+//                     bit for bit.  A group that is already in order, whatever its length, costs
+//                     nothing; one that is out of order and longer than a warp's view sets
+//                     settle_fail, and the plain passes over every digit then sort the array as it
+//                     stands: still a stable arrangement of the input, with the same histograms.
+// Everything is decided on the device, so a sort still never synchronises with the host.
+#pragma once
+#include "rsbd8g_device.cuh"
+
+namespace rsbd8g {
+
+struct PlanArgs {
+    uint64_t spin_limit_ns;
+    uint32_t inplace;      // radixsort / radixsortnoalloc: sort `in` using `buf`
+    uint32_t to_buffer;    // movetobuffer
+    uint32_t rev;          // effective isrevorder
+    uint32_t indirect;
+    uint32_t stall_tile;
+    uint32_t passes;       // digits of the key
+    uint32_t prefetch;     // every array is device memory (Control::prefetch)
+    uint32_t hot_ok;       // crowded digits may be ranked with ballots (PassPlan::hot)
+    uint32_t prefix_ok;    // the launches of a prefix sort follow (slots before and after k_settle)
+};
+
+// The settle step compares a key with its whole group, so its work grows with the group size: up to
+// this many equal-prefix keys on average are left to it.
+constexpr uint64_t kSettleGroup = 2;
+// the copies of one key that are walked over when the sample's pairs are counted
+constexpr uint32_t kSampleRun = 32;
+
+// Every CTA of the histogram launch sorts one key per thread, drawn at random places (independent
+// draws, so an input that is already in order is judged as any other), and counts the pairs of
+// neighbours that differ, weighted with the copies each of the two has, by the highest digit in which
+// they differ.  Many small samples tell as much about equal prefixes as one large one of as many
+// pairs, and sort side by side: a bitonic network, by shuffles within a warp and through shared memory
+// beyond (one 8192-key sample on a CTA of its own took 70 us; these take 3).
+// The pairs that a sample can form should outnumber the keys, for one pair too many to show: a round of
+// samples for every 2^26 keys (152 samples of 1024 keys form 80 M pairs)
+__device__ __forceinline__ uint32_t prefix_rounds(uint64_t n) {
+    const uint64_t r = n >> 26;
+    return r < 1 ? 1u : r > 16 ? 16u : uint32_t(r);
+}
+template <typename U>
+__device__ __forceinline__ U shfl_key(U k, int mask) { return __shfl_xor_sync(0xFFFFFFFFu, k, mask); }
+template <int HB>
+__device__ __forceinline__ KeyWide<HB> shfl_key(KeyWide<HB> k, int mask) {
+    return KeyWide<HB>{__shfl_xor_sync(0xFFFFFFFFu, k.lo, mask), __shfl_xor_sync(0xFFFFFFFFu, k.hi, mask)};
+}
+template <typename U>
+__device__ __forceinline__ U shfl_up_key(U k) { return __shfl_up_sync(0xFFFFFFFFu, k, 1); }
+template <int HB>
+__device__ __forceinline__ KeyWide<HB> shfl_up_key(KeyWide<HB> k) {
+    return KeyWide<HB>{__shfl_up_sync(0xFFFFFFFFu, k.lo, 1), __shfl_up_sync(0xFFFFFFFFu, k.hi, 1)};
+}
+template <typename U>
+__device__ __forceinline__ U shfl_down_key(U k) { return __shfl_down_sync(0xFFFFFFFFu, k, 1); }
+template <int HB>
+__device__ __forceinline__ KeyWide<HB> shfl_down_key(KeyWide<HB> k) {
+    return KeyWide<HB>{__shfl_down_sync(0xFFFFFFFFu, k.lo, 1), __shfl_down_sync(0xFFFFFFFFu, k.hi, 1)};
+}
+template <typename U, int THREADS, typename F>
+__device__ __forceinline__ void prefix_sample(U *s, uint64_t n, Control *__restrict__ ctrl, F key) {
+    static_assert((THREADS & (THREADS - 1)) == 0, "a bitonic network of one key per thread");
+    __shared__ uint32_t pairs[kMaxPasses];
+    const int i = threadIdx.x;
+    if (i < kMaxPasses) pairs[i] = 0;
+    for (uint32_t round = 0; round < prefix_rounds(n); ++round) {
+        // splitmix64 of the sample's index
+        uint64_t z = ((uint64_t(round) * gridDim.x + blockIdx.x) * THREADS + i + 1u) * 0x9E3779B97F4A7C15ull;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        U a = key(__umul64hi(z ^ (z >> 31), n));
+        for (int k = 2; k <= THREADS; k <<= 1) {
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                U b;
+                if (j >= 32) {
+                    __syncthreads();
+                    s[i] = a;
+                    __syncthreads();
+                    b = s[i ^ j];
+                } else {
+                    b = shfl_key(a, j);
+                }
+                const bool low = ((i & j) == 0) == ((i & k) == 0);      // this thread keeps the smaller key
+                if (low ? key_less(b, a) : key_less(a, b)) a = b;
+            }
+        }
+        __syncthreads();
+        s[i] = a;
+        __syncthreads();
+        if (i > 0 && !key_same(s[i - 1], a)) {
+            uint32_t before = 1, after = 1;
+            while (before < kSampleRun && i - 1 - int(before) >= 0 && key_same(s[i - 1 - int(before)], s[i - 1])) ++before;
+            while (after < kSampleRun && i + int(after) < THREADS && key_same(s[i + int(after)], a)) ++after;
+            atomicAdd(pairs + top_diff(s[i - 1], a), before * after);
+        }
+        __syncthreads();                                               // s is free again
+    }
+    if (i < kMaxPasses && pairs[i]) atomicAdd(&ctrl->sample_pairs[i], pairs[i]);
+}
+
+// The passes of the shortest prefix that leaves groups of about kSettleGroup keys or fewer, *low its
+// lowest digit; 0 for a plain sort.  W pairs of a sample that can form `all` pairs stand for n W / all
+// other keys with the same prefix per key.  One thread calls it.
+__device__ __forceinline__ uint32_t prefix_choose(const uint32_t *sample_pairs, uint32_t survive, uint64_t n, uint64_t all,
+                                                  uint32_t *low) {
+    const int digits = __popc(survive);
+    uint64_t pairs = 0;
+    uint32_t k = 0;
+    for (int q = 0; q < kMaxPasses && pairs < (1u << 20); ++q) {   // pairs: their highest differing digit is below q
+        if ((survive >> q) & 1u) {
+            const int passes = __popc(survive >> q);
+            // at least two passes must be saved: the settle step reads every key once
+            if (passes <= kPrefixSlots && passes <= digits - 2 && (pairs + 1u) * n <= kSettleGroup * all) {
+                k = uint32_t(passes);
+                *low = uint32_t(q);
+            }
+        }
+        pairs += sample_pairs[q];
+    }
+    return k;
+}
+
+// Plan the passes over the digits of `mask`, lowest first, from array `cur` on; returns where they
+// end.  Launch slots: keys of up to 4 bytes take the slot of the digit's number, wider keys consecutive
+// slots from slot0.  A copy form must end in its output; `even` makes the number of passes even (by
+// sorting by the lowest digit twice) for a chain that starts there.  keep_keys: the last pass of an
+// indirect sort writes its keys too; hot: the crowded digit of each position.  One thread calls it.
+__device__ __forceinline__ uint32_t plan_chain(Control *__restrict__ ctrl, const PlanArgs &a, const uint32_t *hot, uint32_t mask, bool even,
+                                               int slot0, uint32_t cur, uint32_t &curk, bool rev, bool keep_keys) {
+    const int again = even && (__popc(mask) & 1) ? 1 : 0;
+    const int k = __popc(mask) + again;
+    int p = -1;
+    for (int i = 1; i <= k; ++i) {
+        if (!(again && i == 2)) {
+            do ++p;
+            while (!((mask >> p) & 1u));
+        }
+        const int slot = a.passes >= 8 ? slot0 + i - 1 : p;
+        PassPlan &pp = ctrl->plan[slot];
+        pp.active = 1u;
+        pp.hot = hot[p];
+        pp.digit = uint16_t(p);
+        pp.status = uint16_t(a.passes >= 8 ? i - 1 : p);
+        uint32_t dst;
+        if (a.inplace) dst = (cur == kArrIn) ? kArrBuf : kArrIn;
+        else dst = ((k - i) % 2 == 0) ? kArrOut : kArrBuf;
+        pp.reverse = (i == 1) && rev;
+        if (a.indirect) {
+            pp.src_vals = cur;
+            pp.dst_vals = dst;
+            pp.src_keys = curk;
+            const uint32_t dk = (curk == kArrKeysA) ? kArrKeysB : kArrKeysA;
+            pp.dst_keys = (i == k && !keep_keys) ? kArrNone : dk;
+            curk = dk;
+        } else {
+            pp.src_keys = cur;
+            pp.dst_keys = dst;
+            pp.src_vals = kArrNone;
+            pp.dst_vals = kArrNone;
+        }
+        cur = dst;
+    }
+    return cur;
+}
+
+// The copy step after passes that end in array `cur` (no_pass: none of them runs, so a reversal of
+// the order is still to be done).  One thread calls it.
+__device__ __forceinline__ void plan_copy(Control *__restrict__ ctrl, const PlanArgs &a, uint32_t cur, bool no_pass) {
+    ctrl->copy_mode = kCopyNone;
+    if (!a.inplace) {
+        if (no_pass) {
+            ctrl->copy_mode = a.rev ? kCopyReversed : kCopyPlain;
+            ctrl->copy_src = kArrIn;
+            ctrl->copy_dst = kArrOut;
+        }
+    } else {
+        const uint32_t target = a.to_buffer ? kArrBuf : kArrIn;
+        if (no_pass && a.rev) {
+            ctrl->copy_mode = a.to_buffer ? kCopyReversed : kReverseInPlace;
+            ctrl->copy_src = kArrIn;
+            ctrl->copy_dst = target;
+        } else if (cur != target) {
+            ctrl->copy_mode = kCopyPlain;
+            ctrl->copy_src = cur;
+            ctrl->copy_dst = target;
+        }
+    }
+}
+
+// ---- the settle step ---------------------------------------------------------------------------
+// Warps take chunks in turn, each on its own (no barrier, so many warps' loads are in flight).  A lane
+// holds kItems neighbouring keys in registers; the last lane's keys are the halo, the first keys of
+// the next chunk.  A key is a head if its prefix differs from the one before it, else an inversion if
+// it is below the key before it.  A group belongs to the chunk it starts in, and is put in order by rounds
+// of exchanges between neighbours of one group (only a key below the one before it passes it, so equal
+// keys keep their order): a round per key that another has to pass, a few for groups of a few keys.
+//   A group that is still open at the end of the halo, or takes more than kRounds rounds, is settled by
+// the warp in shared memory, with kView keys in view, every key moving to the place found by comparing
+// it with its group.  A group from an earlier chunk is left alone, so an inversion in one raises
+// settle_fail unless the chunk before this one holds its start and this one's first kReach keys hold
+// the inversion; and so does an inversion in a group that runs past kView.  So no inversion is passed over.
+// Neighbouring chunks read keys that a chunk moves only for their prefixes, which a move within a
+// group leaves as they are.
+template <typename U>
+struct SettleShape {
+    static constexpr int kThreads = sizeof(U) == 8 ? 256 : 128;     // (static shared memory stays below 48 KB)
+    static constexpr int kWarps = kThreads / 32;
+    static constexpr int kItems = 8;
+    static constexpr int kChunk = 31 * kItems;
+    static constexpr int kCtaKeys = kWarps * kChunk;
+    static constexpr int kReach = 224;
+    static constexpr int kView = kChunk + kReach;
+    static constexpr int kWords = (kView + 31) / 32;
+    static constexpr int kRounds = 12;
+};
+
+// the last set bit of w[] at or below position i, -1 if there is none
+__device__ __forceinline__ int bit_at_or_below(const uint32_t *w, int i) {
+    int x = i >> 5;
+    uint32_t m = w[x] & (0xFFFFFFFFu >> (31 - (i & 31)));
+    while (!m && --x >= 0) m = w[x];
+    return m ? x * 32 + 31 - __clz(m) : -1;
+}
+// the first set bit of w[0, words) at or above position i, words * 32 if there is none
+__device__ __forceinline__ int bit_at_or_above(const uint32_t *w, int i, int words) {
+    int x = i >> 5;
+    if (x >= words) return words * 32;
+    uint32_t m = w[x] & (0xFFFFFFFFu << (i & 31));
+    while (!m && ++x < words) m = w[x];
+    return m ? x * 32 + __ffs(m) - 1 : words * 32;
+}
+
+// ITEMS keys from p on: 16-byte loads where the address allows
+template <int ITEMS, typename U>
+__device__ __forceinline__ void load_run(U (&v)[ITEMS], const U *p) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+        constexpr int V = 16 / int(sizeof(U));
+#pragma unroll
+        for (int i = 0; i < ITEMS; i += V) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(p + i);
+            memcpy(&v[i], &q, 16);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) v[i] = p[i];
+    }
+}
+
+// the key as the sort orders it
+template <int MODE, typename U>
+__device__ __forceinline__ U settle_order(U b, bool desc) {
+    const U q = filter_key<MODE>(b);
+    return desc ? key_not(q) : q;
+}
+
+// one warp settles the groups that start in the chunk at c0, in shared memory
+template <int MODE, bool HAS_VAL, typename S, typename U>
+__device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, U *key,
+                                         uint32_t *hw, uint32_t *vw, uint32_t *fail) {
+    constexpr int WORDS = S::kWords;
+    const int lane = int(threadIdx.x & 31u);
+    const int view = int(n - c0 < uint64_t(S::kView) ? n - c0 : uint64_t(S::kView));
+    for (int x = lane; x < view; x += 32) key[x] = keys[c0 + x];
+    __syncwarp();
+    for (int w = 0; w < WORDS; ++w) {
+        const int x = w * 32 + lane;
+        bool h = x == 0 ? c0 == 0 : x >= view, v = false;
+        if (!h) {
+            const U a = settle_order<MODE>(x ? key[x ? x - 1 : 0] : keys[c0 - 1], desc), b = settle_order<MODE>(key[x], desc);
+            h = !same_masked(a, b, mask);
+            v = !h && key_less(b, a);
+        }
+        const uint32_t hm = __ballot_sync(0xFFFFFFFFu, h), vm = __ballot_sync(0xFFFFFFFFu, v);
+        if (lane == 0) {
+            hw[w] = hm;
+            vw[w] = vm;
+        }
+    }
+    __syncwarp();
+    int s = bit_at_or_above(hw, 0, WORDS);                // the first group that starts here
+    while (s < S::kChunk && s < view) {
+        const int x = bit_at_or_above(vw, s, WORDS);      // the next inversion, and its group
+        if (x >= view) break;
+        s = bit_at_or_below(hw, x);
+        if (s >= S::kChunk) break;
+        int e = bit_at_or_above(hw, x + 1, WORDS);
+        if (e >= view) {
+            if (c0 + uint64_t(view) < n) {                // it runs on past the view
+                if (lane == 0) atomicOr(fail, 1u);
+                break;
+            }
+            e = view;
+        }
+        uint64_t p[HAS_VAL ? WORDS : 1];
+        if constexpr (HAS_VAL) {                          // every pointer of the group is read before any is moved
+            for (int i = s + lane, r = 0; i < e; i += 32, ++r) p[r] = vals[c0 + i];
+            __syncwarp();
+        }
+        for (int i = s + lane, r = 0; i < e; i += 32, ++r) {
+            const U b = settle_order<MODE>(key[i], desc);
+            int at = s;
+            for (int j = s; j < e; ++j) {
+                const U a = settle_order<MODE>(key[j], desc);
+                at += key_less(a, b) || (j < i && key_same(a, b)) ? 1 : 0;
+            }
+            keys[c0 + at] = key[i];
+            if constexpr (HAS_VAL) vals[c0 + at] = p[r];
+        }
+        s = e;
+    }
+    __syncwarp();                                         // the warp's shared memory is free again
+}
+
+template <typename U, int MODE, bool HAS_VAL>
+__global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HAS_VAL ? 4 : 5) : 6)
+    k_settle(Control *__restrict__ ctrl, const SortArrays arrs, uint64_t n, uint32_t desc, unsigned char *status,
+             size_t status_bytes, PlanArgs pa) {
+    using S = SettleShape<U>;
+    constexpr int THREADS = S::kThreads, ITEMS = S::kItems, C = S::kChunk;
+    const uint32_t k = ctrl->prefix_passes;
+    if (k == 0 || ctrl->abort) return;
+    __shared__ __align__(16) U keys_s[S::kWarps][S::kView];
+    __shared__ uint32_t words_s[S::kWarps][2][S::kWords];
+    __shared__ uint32_t last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const PassPlan &end = ctrl->plan[k - 1];
+    bool bad = false;
+    U *keys = static_cast<U *>(sort_array(arrs, end.dst_keys, HAS_VAL ? kArrKeysA : kArrBuf, &bad));
+    uint64_t *vals = static_cast<uint64_t *>(sort_array(arrs, end.dst_vals, kArrBuf, &bad));
+    if (bad || !keys || (HAS_VAL && !vals)) {       // a damaged control block
+        if (tid == 0) atomicOr(&ctrl->error, kDevFault);
+        return;
+    }
+    // the prefix passes' look-back words, cleared for the plain passes that a failure calls for
+    for (uint64_t i = uint64_t(blockIdx.x) * THREADS + tid; i < uint64_t(k) * status_bytes / 16; i += uint64_t(gridDim.x) * THREADS)
+        reinterpret_cast<uint4 *>(status)[i] = make_uint4(0, 0, 0, 0);
+    const U mask = prefix_mask<U>(ctrl->prefix_low);
+    const uint64_t chunks = (n + C - 1) / C, stride = uint64_t(gridDim.x) * S::kWarps;
+    uint32_t seen = 0;
+    for (uint64_t c = uint64_t(blockIdx.x) * S::kWarps + warp; c < chunks; c += stride) {
+        // the failure flag is one word for the whole grid: looked at now and then
+        if ((++seen & 15u) == 0 && ld_relaxed(&ctrl->settle_fail)) break;
+        const uint64_t c0 = c * C;
+        const bool full = n - c0 >= uint64_t(32 * ITEMS);
+        const int own = full ? ITEMS : int(n - c0) - lane * ITEMS;      // this lane's keys (may be < 0 or > ITEMS)
+        U v[ITEMS], before{};
+        if (full) {
+            load_run<ITEMS>(v, keys + c0 + lane * ITEMS);
+        } else {
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) {
+                v[j] = U{};
+                if (j < own) v[j] = keys[c0 + lane * ITEMS + j];
+            }
+        }
+        if (lane == 0 && c0) before = keys[c0 - 1];
+        // heads and inversions among this lane's keys (bit j: key j)
+        uint32_t hb = 0, vb = 0;
+        {
+            const U up = shfl_up_key(v[ITEMS - 1]);
+            U a = settle_order<MODE>(lane ? up : before, desc);
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) {
+                const U b = settle_order<MODE>(v[j], desc);
+                const bool h = !same_masked(a, b, mask);
+                if (h) hb |= 1u << j;
+                else if (key_less(b, a)) vb |= 1u << j;
+                a = b;
+            }
+        }
+        if (c0 == 0 && lane == 0) hb |= 1u;
+        if (!full) hb |= own >= ITEMS ? 0u : own <= 0 ? 0xFFu : 0xFFu << own;     // past the end: each alone
+        vb &= ~hb;
+        const uint32_t heads = __ballot_sync(0xFFFFFFFFu, hb != 0);
+        const bool open = !(heads >> 31) && (heads & 0x7FFFFFFFu) && n - c0 > uint64_t(32 * ITEMS);
+        if (!__any_sync(0xFFFFFFFFu, vb != 0) && !open) continue;
+        // this lane's keys of the group that came in, and of the groups that the next chunk settles
+        const uint32_t below = hb ? (hb & (0u - hb)) - 1u : 0xFFu;      // keys before the lane's first head
+        const uint32_t in = (heads & ((1u << lane) - 1u)) == 0 ? below : 0u;
+        const uint32_t out = lane == 31 ? ~below & 0xFFu : 0u;
+        const uint32_t bad_in = vb & in;
+        if (__any_sync(0xFFFFFFFFu, bad_in != 0)) {
+            // settled by the chunk before, if it holds the start and sees the inversion
+            bool lost = bad_in && lane * ITEMS + 31 - __clz(bad_in) >= S::kReach;
+            if (bad_in && c0 > uint64_t(C)) {
+                const U a = settle_order<MODE>(keys[c0 - C - 1], desc), b = settle_order<MODE>(keys[c0 - 1], desc);
+                lost |= same_masked(a, b, mask);
+            }
+            if (lost) atomicOr(&ctrl->settle_fail, 1u);
+        }
+        const uint32_t pass = ~hb & ~in & ~out & 0xFFu;          // keys that may pass the one before them
+        bool wide = open;
+        if (!open) {
+            uint32_t moved = 0, from[HAS_VAL ? ITEMS : 1];
+            if constexpr (HAS_VAL) {
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j) from[j] = uint32_t(lane * ITEMS + j);
+            }
+            const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, pass, 1);
+            const bool pass0 = (pass & 1u) && lane, pass8 = lane < 31 && (next & 1u);
+            // one round settles a chunk whose groups have two keys at most
+            const bool several = __any_sync(0xFFFFFFFFu, (pass & (pass << 1)) != 0 || (pass8 && (pass >> (ITEMS - 1))));
+            for (int r = 0;; ++r) {
+                bool swapped = false;
+                // across the lanes: both sides see the same two keys and come to the same answer
+                const U up = shfl_up_key(v[ITEMS - 1]), down = shfl_down_key(v[0]);
+                uint32_t fup = 0, fdown = 0;
+                if constexpr (HAS_VAL) {
+                    fup = __shfl_up_sync(0xFFFFFFFFu, from[ITEMS - 1], 1);
+                    fdown = __shfl_down_sync(0xFFFFFFFFu, from[0], 1);
+                }
+                if (pass0 && key_less(settle_order<MODE>(v[0], desc), settle_order<MODE>(up, desc))) {
+                    v[0] = up;
+                    if constexpr (HAS_VAL) from[0] = fup;
+                    moved |= 1u;
+                    swapped = true;
+                }
+                if (pass8 && key_less(settle_order<MODE>(down, desc), settle_order<MODE>(v[ITEMS - 1], desc))) {
+                    v[ITEMS - 1] = down;
+                    if constexpr (HAS_VAL) from[HAS_VAL ? ITEMS - 1 : 0] = fdown;
+                    moved |= 1u << (ITEMS - 1);
+                    swapped = true;
+                }
+#pragma unroll
+                for (int j = 1; j < ITEMS; ++j) {
+                    if (((pass >> j) & 1u) && key_less(settle_order<MODE>(v[j], desc), settle_order<MODE>(v[j - 1], desc))) {
+                        const U t = v[j];
+                        v[j] = v[j - 1];
+                        v[j - 1] = t;
+                        if constexpr (HAS_VAL) {
+                            const uint32_t f = from[HAS_VAL ? j : 0];
+                            from[HAS_VAL ? j : 0] = from[HAS_VAL ? j - 1 : 0];
+                            from[HAS_VAL ? j - 1 : 0] = f;
+                        }
+                        moved |= 3u << (j - 1);
+                        swapped = true;
+                    }
+                }
+                if (!several || !__any_sync(0xFFFFFFFFu, swapped)) break;
+                if (r == S::kRounds) {
+                    wide = true;
+                    break;
+                }
+            }
+            if (!wide) {
+                U *dst = keys + c0 + lane * ITEMS;
+                if constexpr (HAS_VAL) {
+                    uint64_t p[ITEMS];
+#pragma unroll
+                    for (int j = 0; j < ITEMS; ++j)
+                        if ((moved >> j) & 1u) p[j] = vals[c0 + from[j]];
+                    __syncwarp();                    // every pointer that moves has been read
+#pragma unroll
+                    for (int j = 0; j < ITEMS; ++j)
+                        if ((moved >> j) & 1u) vals[c0 + lane * ITEMS + j] = p[j];
+                }
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j)
+                    if ((moved >> j) & 1u) dst[j] = v[j];
+            }
+        }
+        if (wide)
+            settle_wide<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc != 0, keys_s[warp], words_s[warp][0],
+                                          words_s[warp][1], &ctrl->settle_fail);
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(&ctrl->settle_done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!last || tid != 0 || !ld_relaxed(&ctrl->settle_fail)) return;
+    // a group was too long to settle: the plain passes, over every digit, from where the data stand
+    const uint32_t cur = HAS_VAL ? end.dst_vals : end.dst_keys;
+    uint32_t curk = end.dst_keys;
+    const uint32_t done = plan_chain(ctrl, pa, ctrl->hot, ctrl->survive, !pa.inplace, kPrefixSlots, cur, curk, false, false);
+    plan_copy(ctrl, pa, done, false);
+}
+
+}  // namespace rsbd8g
