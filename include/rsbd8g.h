@@ -324,7 +324,7 @@ RSBD8G_API const char *rsbd8g_status_string(rsbd8g_status status);
 enum {
     RSBD8G_KERNEL_MEMSET = 0, RSBD8G_KERNEL_HISTOGRAM = 1, RSBD8G_KERNEL_PLAN = 2,
     RSBD8G_KERNEL_ONESWEEP = 3, RSBD8G_KERNEL_COPY = 4, RSBD8G_KERNEL_SEGMENTED = 5, RSBD8G_KERNEL_MERGE = 6,
-    RSBD8G_KERNEL_SETTLE = 7
+    RSBD8G_KERNEL_SETTLE = 7, RSBD8G_KERNEL_ONE = 8
 };
 
 typedef struct rsbd8g_launch_record {

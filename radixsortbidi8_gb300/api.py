@@ -65,7 +65,7 @@ EXPORTS = ["rsbd8g_scratch_bytes", "rsbd8g_radixsortcopy", "rsbd8g_radixsort",
            "rsbd8g_radixsortcopynoalloc", "rsbd8g_radixsortnoalloc", "rsbd8g_scratch_status",
            "rsbd8g_status_string", "rsbd8g_version", "rsbd8g_profile_enable", "rsbd8g_profile_collect"]
 
-KERNEL_NAMES = {0: "memset", 1: "histogram", 2: "plan", 3: "onesweep", 4: "copy", 5: "segmented", 6: "merge", 7: "settle"}
+KERNEL_NAMES = {0: "memset", 1: "histogram", 2: "plan", 3: "onesweep", 4: "copy", 5: "segmented", 6: "merge", 7: "settle", 8: "one"}
 
 
 class LaunchRecord(ctypes.Structure):

@@ -210,12 +210,7 @@ bool device_memory(const void *p) {
 
 rsbd8g_status enqueue_sort(const Resolved &rin, uint64_t n, void *scratch, size_t scratch_bytes, const void *in,
                            void *out, void *buf, bool inplace, bool to_buffer, cudaStream_t s) {
-    // the scatter passes prefetch tiles into L2 with bulk copies only from device memory
-    // (cudaMalloc, memory pools); managed and host memory is read with plain loads alone
     Resolved r = rin;
-    r.prefetch = (r.flags & RSBD8G_FLAG_DEVICE_ARRAYS) ||
-                 (device_memory(in) && device_memory(out) && device_memory(buf) &&
-                  (!r.indirect || device_memory(scratch)));
     if (n > kMaxCount) return RSBD8G_ERR_TOO_LARGE;
     const Layout L = layout_for(r, n);
     if (!scratch || scratch_bytes < L.total) return RSBD8G_ERR_BAD_ARG;
@@ -225,7 +220,24 @@ rsbd8g_status enqueue_sort(const Resolved &rin, uint64_t n, void *scratch, size_
         auto mis = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) != 0; };
         if (mis(in) || (out && mis(out)) || (buf && mis(buf))) return RSBD8G_ERR_BAD_ARG;
     }
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
+    bool one;           // a small sort runs as one kernel
+    switch (r.key_bytes) {
+        case 1: one = launch_one_k1(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
+        case 2: one = launch_one_k2(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
+        case 4: one = launch_one_k4(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
+        case 8: one = launch_one_k8(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
+        default:
+            one = r.x87 ? launch_one_x87(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e)
+                        : launch_one_k16(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e);
+            break;
+    }
+    if (one) return e == cudaSuccess ? RSBD8G_OK : RSBD8G_ERR_CUDA;
+    // the scatter passes prefetch tiles into L2 with bulk copies only from device memory
+    // (cudaMalloc, memory pools); managed and host memory is read with plain loads alone
+    r.prefetch = (r.flags & RSBD8G_FLAG_DEVICE_ARRAYS) ||
+                 (device_memory(in) && device_memory(out) && device_memory(buf) &&
+                  (!r.indirect || device_memory(scratch)));
     switch (r.key_bytes) {
         case 1: e = launch_sort_k1(r, n, L, sc, in, out, buf, inplace, to_buffer, s); break;
         case 2: e = launch_sort_k2(r, n, L, sc, in, out, buf, inplace, to_buffer, s); break;
@@ -286,6 +298,13 @@ RSBD8G_API rsbd8g_status rsbd8g_prepare(const rsbd8g_desc *desc) {
     if (st != RSBD8G_OK) return st;
     cudaError_t e;
     switch (r.key_bytes) {
+        case 1: e = launch_one_k1_prepare(r); break;
+        case 2: e = launch_one_k2_prepare(r); break;
+        case 4: e = launch_one_k4_prepare(r); break;
+        case 8: e = launch_one_k8_prepare(r); break;
+        default: e = r.x87 ? launch_one_x87_prepare(r) : launch_one_k16_prepare(r); break;
+    }
+    if (e == cudaSuccess) switch (r.key_bytes) {
         case 1: e = launch_sort_k1_prepare(r); break;
         case 2: e = launch_sort_k2_prepare(r); break;
         case 4: e = launch_sort_k4_prepare(r); break;

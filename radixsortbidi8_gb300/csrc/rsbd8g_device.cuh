@@ -281,6 +281,16 @@ __device__ __forceinline__ void st_relaxed(uint64_t *p, uint64_t v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// loads that another CTA's writes of the same launch reach (past L1)
+template <typename U>
+__device__ __forceinline__ U ld_l2(const U *p) { return __ldcg(p); }
+__device__ __forceinline__ uint64_t ld_l2(const uint64_t *p) { return __ldcg(reinterpret_cast<const unsigned long long *>(p)); }
+template <int HB>
+__device__ __forceinline__ KeyWide<HB> ld_l2(const KeyWide<HB> *p) {
+    const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(p));
+    return KeyWide<HB>{v.x, v.y};
+}
+
 // status word helpers: state in the top two bits, count below
 template <typename S> struct StatusWord;
 template <> struct StatusWord<uint32_t> {

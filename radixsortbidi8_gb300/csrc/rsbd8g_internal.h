@@ -62,6 +62,20 @@ RSBD8G_DECLARE_LAUNCH(launch_sort_k8)
 RSBD8G_DECLARE_LAUNCH(launch_sort_k16)
 RSBD8G_DECLARE_LAUNCH(launch_sort_x87)
 
+// the one-kernel sorts of small arrays, per key size (rsbd8g_one_k*.cu): false (nothing launched) when
+// the sort does not fit one
+#define RSBD8G_DECLARE_ONE(name)                                                                             \
+    bool name(const Resolved &r, uint64_t n, unsigned char *scratch, size_t scratch_bytes, const void *in,   \
+              void *out, void *buf, const Layout &L, bool inplace, bool to_buffer, cudaStream_t s,           \
+              cudaError_t *e);                                                                               \
+    cudaError_t name##_prepare(const Resolved &r);
+RSBD8G_DECLARE_ONE(launch_one_k1)
+RSBD8G_DECLARE_ONE(launch_one_k2)
+RSBD8G_DECLARE_ONE(launch_one_k4)
+RSBD8G_DECLARE_ONE(launch_one_k8)
+RSBD8G_DECLARE_ONE(launch_one_k16)
+RSBD8G_DECLARE_ONE(launch_one_x87)
+
 // tile geometry of the onesweep passes, per key size (keys per tile = threads * items)
 struct SweepGeometry {
     int threads, items;

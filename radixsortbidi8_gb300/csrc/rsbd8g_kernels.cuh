@@ -433,7 +433,8 @@ struct TileRank {
 
     // rank this lane's ITEMS keys within its unit (the unit's masks clear, its counts zero); with
     // HOT > 0 the digits in `hot` ((digit1 << 16) | digit0, kNoHot for none) are ranked by ballots
-    template <int MODE, int HOT = 0, typename U>
+    // (PADS false: padding slots are left out of the table, and get no rank)
+    template <int MODE, int HOT = 0, bool PADS = true, typename U>
     __device__ static void rank(const U (&keys)[ITEMS], uint32_t (&rk)[kRankRegs], uint32_t *tab, uint32_t slot0,
                                 uint32_t tvalid, int pass, uint32_t dmask, uint32_t hot = kNoHotPair) {
         uint32_t *crow = row(tab);
@@ -446,7 +447,7 @@ struct TileRank {
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
             const uint32_t d = slot_digit<MODE>(keys[i], slot0 + uint32_t(LANES) * i, tvalid, pass, dmask);
-            bool is_hot = false;
+            bool is_hot = !PADS && slot0 + uint32_t(LANES) * i >= tvalid;
             uint32_t rh = 0;
             if constexpr (HOT > 0) {
                 const uint32_t b0 = (__ballot_sync(0xFFFFFFFFu, d == h0) >> ushift) & umask;
