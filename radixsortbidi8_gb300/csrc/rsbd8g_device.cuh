@@ -222,6 +222,13 @@ __host__ __device__ __forceinline__ KeyWide<HB> filter_key(KeyWide<HB> b) {
     }
 }
 
+// Programmatic dependent launch: a kernel launched with launch_after starts while the kernel before it
+// in the stream drains.  after_previous() waits until that kernel has ended and its writes are visible
+// (at once in a launch without the attribute): nothing in global memory is touched before it.
+// next_may_start() lets the following kernel's CTAs take the places that come free.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // order, equality and digit comparisons of filtered keys
 template <typename U>
 __host__ __device__ __forceinline__ bool key_less(U a, U b) { return a < b; }

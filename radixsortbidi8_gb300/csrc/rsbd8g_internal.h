@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <type_traits>
 
 #include "rsbd8g.h"
 #include "rsbd8g_device.cuh"
@@ -49,6 +50,23 @@ private:
 };
 
 int device_sms(int dev);
+
+// launch a kernel that calls after_previous(): it may start while the stream's previous kernel drains
+template <typename... A>
+cudaError_t launch_after(void (*kern)(A...), uint32_t grid, int threads, size_t smem, cudaStream_t s,
+                         std::common_type_t<A>... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(unsigned(threads));
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, args...);
+}
 
 // the launch sequence of one sort, per key size (rsbd8g_sort_k{1,2,4,8}.cu)
 #define RSBD8G_DECLARE_LAUNCH(name)                                                                          \

@@ -172,6 +172,7 @@ __device__ __forceinline__ void plan_if_last(Control *__restrict__ ctrl, const u
                                              unsigned long long *__restrict__ bstart, uint64_t n, const PlanArgs &a) {
     static_assert(THREADS >= kBuckets && THREADS % 32 == 0, "the plan needs a thread per digit");
     __shared__ uint32_t last;
+    next_may_start();
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(&ctrl->hist_done, 1u) == gridDim.x - 1 ? 1u : 0u;
@@ -345,6 +346,7 @@ __device__ __forceinline__ void copy_step(Control *__restrict__ ctrl, const Sort
 // the copy step of the in-place forms, after the last pass
 static __global__ void __launch_bounds__(256) k_copy(Control *__restrict__ ctrl, const SortArrays arrs, uint64_t n,
                                                      uint32_t elem_bytes) {
+    after_previous();
     copy_step(ctrl, arrs, n, elem_bytes);
 }
 
@@ -866,6 +868,8 @@ __global__ void __launch_bounds__(THREADS, onesweep_min_blocks<U, HAS_VAL, THREA
     static_assert(THREADS >= kBuckets && THREADS % 32 == 0, "one thread per digit");
     static_assert(L::kTile <= 65535, "tile ranks are 16-bit");
     extern __shared__ __align__(16) unsigned char smem[];
+    next_may_start();
+    after_previous();
     const PassPlan plan = ctrl->plan[slot];
     if (!plan.active) {
         // the last pass of a copy form: when every pass was skipped, the copy the plan asks for
@@ -1125,6 +1129,8 @@ __global__ void __launch_bounds__(THREADS, 2)
     static_assert(THREADS == 2 * kBuckets, "threads 0..255 scan, threads 256..511 look back");
     static_assert(PipeSmem<U, THREADS, ITEMS, HAS_VAL>::kTile <= 65535, "tile ranks are 16-bit");
     extern __shared__ __align__(16) unsigned char smem[];
+    next_may_start();
+    after_previous();
     const PassPlan plan = ctrl->plan[slot];
     if (!plan.active) {
         // the last pass of a copy form: when every pass was skipped, the copy the plan asks for

@@ -70,9 +70,9 @@ cudaError_t launch_settle_t(uint64_t n, const Layout &L, unsigned char *scratch,
     cudaGetDevice(&dev);
     const uint64_t tiles = (n + SettleShape<U>::kCtaKeys - 1) / SettleShape<U>::kCtaKeys;
     const uint64_t resident = uint64_t(settle_setup<U, MODE, HAS_VAL>(dev)) * device_sms(dev);
-    k_settle<U, MODE, HAS_VAL><<<uint32_t(std::min(tiles, resident)), SettleShape<U>::kThreads, 0, s>>>(
-        reinterpret_cast<Control *>(scratch + L.ctrl), arrs, n, dmask, scratch + L.status, L.status_pass_bytes, pa);
-    return cudaGetLastError();
+    return launch_after(k_settle<U, MODE, HAS_VAL>, uint32_t(std::min(tiles, resident)), SettleShape<U>::kThreads, 0, s,
+                        reinterpret_cast<Control *>(scratch + L.ctrl), arrs, n, dmask, scratch + L.status,
+                        L.status_pass_bytes, pa);
 }
 
 template <typename U, int MODE, bool HAS_VAL, int THREADS, int ITEMS, typename S>
@@ -110,9 +110,9 @@ cudaError_t launch_sweeps_t(uint32_t passes, uint64_t n, const Layout &L, unsign
         S *st = status + (KeyTraits<U>::kDigits >= 8 ? 0 : size_t(p) * stride);
         const uint32_t fc = (fold_copy && p + 1 == slots) ? 1u : 0u;   // the copy forms' copy, in the last pass
         if (pipe)
-            pkern<<<grid, THREADS, PM::kBytes, s>>>(ctrl, arrs, bstart, st, stride, int(p), n, L.num_tiles, dmask, fc);
+            launch_after(pkern, grid, THREADS, PM::kBytes, s, ctrl, arrs, bstart, st, stride, int(p), n, L.num_tiles, dmask, fc);
         else
-            kern<<<grid, THREADS, SM::kBytes, s>>>(ctrl, arrs, bstart, st, stride, int(p), n, L.num_tiles, dmask, fc);
+            launch_after(kern, grid, THREADS, SM::kBytes, s, ctrl, arrs, bstart, st, stride, int(p), n, L.num_tiles, dmask, fc);
     }
     return cudaGetLastError();
 }
@@ -225,7 +225,7 @@ cudaError_t launch_sort_t(const Resolved &r, uint64_t n, const Layout &L, unsign
     const uint32_t cgrid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, uint64_t(device_sms(dev)) * 8)));
     {
         LaunchTimer t(s, RSBD8G_KERNEL_COPY, uint32_t(sizeof(U)), 0, n);
-        k_copy<<<cgrid, 256, 0, s>>>(reinterpret_cast<Control *>(scratch + L.ctrl), arrs, n, uint32_t(r.elem_bytes));
+        launch_after(k_copy, cgrid, 256, 0, s, reinterpret_cast<Control *>(scratch + L.ctrl), arrs, n, uint32_t(r.elem_bytes));
     }
     return cudaGetLastError();
 }

@@ -331,6 +331,8 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
              size_t status_bytes, PlanArgs pa) {
     using S = SettleShape<U>;
     constexpr int THREADS = S::kThreads, ITEMS = S::kItems, C = S::kChunk;
+    next_may_start();
+    after_previous();
     const uint32_t k = ctrl->prefix_passes;
     if (k == 0 || ctrl->abort) return;
     __shared__ __align__(16) U keys_s[S::kWarps][S::kView];
