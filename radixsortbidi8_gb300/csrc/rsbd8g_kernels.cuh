@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(THREADS) k_histogram(const U *__restrict__ key
     extern __shared__ __align__(16) uint32_t shl[];
     if constexpr (P >= 8) {
         if (pa.prefix_ok)
-            prefix_sample<U, THREADS>(reinterpret_cast<U *>(shl), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(keys[i]); });
+            prefix_sample_cta<U, THREADS>(reinterpret_cast<U *>(shl), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(keys[i]); });
     }
     for (int i = threadIdx.x; i < C * P * kBuckets; i += THREADS) shl[i] = 0;
     __syncthreads();
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(THREADS) k_gather_histogram(const uint64_t *__
     };
     if constexpr (P >= 8) {
         if (pa.prefix_ok)
-            prefix_sample<U, THREADS>(reinterpret_cast<U *>(shall), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(key_at(i)); });
+            prefix_sample_cta<U, THREADS>(reinterpret_cast<U *>(shall), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(key_at(i)); });
     }
     zero_hist<THREADS, P>(shall);
     uint32_t *sh = shall + ((threadIdx.x >> 5) % gather_hist_copies<P>()) * P * kBuckets;

@@ -72,14 +72,13 @@ __device__ __forceinline__ KeyWide<HB> shfl_down_key(KeyWide<HB> k) {
     return KeyWide<HB>{__shfl_down_sync(0xFFFFFFFFu, k.lo, 1), __shfl_down_sync(0xFFFFFFFFu, k.hi, 1)};
 }
 template <typename U, int THREADS, typename F>
-__device__ __forceinline__ void prefix_sample(U *s, uint64_t n, Control *__restrict__ ctrl, F key) {
+__device__ __forceinline__ void prefix_sample(U *s, uint64_t n, uint32_t rounds, uint64_t first, uint32_t *pairs, F key) {
     static_assert((THREADS & (THREADS - 1)) == 0, "a bitonic network of one key per thread");
-    __shared__ uint32_t pairs[kMaxPasses];
     const int i = threadIdx.x;
     if (i < kMaxPasses) pairs[i] = 0;
-    for (uint32_t round = 0; round < prefix_rounds(n); ++round) {
+    for (uint32_t round = 0; round < rounds; ++round) {
         // splitmix64 of the sample's index
-        uint64_t z = ((uint64_t(round) * gridDim.x + blockIdx.x) * THREADS + i + 1u) * 0x9E3779B97F4A7C15ull;
+        uint64_t z = ((first + round) * THREADS + i + 1u) * 0x9E3779B97F4A7C15ull;
         z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
         z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
         U a = key(__umul64hi(z ^ (z >> 31), n));
@@ -109,7 +108,14 @@ __device__ __forceinline__ void prefix_sample(U *s, uint64_t n, Control *__restr
         }
         __syncthreads();                                               // s is free again
     }
-    if (i < kMaxPasses && pairs[i]) atomicAdd(&ctrl->sample_pairs[i], pairs[i]);
+}
+// the samples of one histogram CTA, added to the sort's
+template <typename U, int THREADS, typename F>
+__device__ __forceinline__ void prefix_sample_cta(U *s, uint64_t n, Control *__restrict__ ctrl, F key) {
+    __shared__ uint32_t pairs[kMaxPasses];
+    const uint32_t rounds = prefix_rounds(n);
+    prefix_sample<U, THREADS>(s, n, rounds, uint64_t(blockIdx.x) * rounds, pairs, key);
+    if (threadIdx.x < kMaxPasses && pairs[threadIdx.x]) atomicAdd(&ctrl->sample_pairs[threadIdx.x], pairs[threadIdx.x]);
 }
 
 // The passes of the shortest prefix that leaves groups of about kSettleGroup keys or fewer, *low its
@@ -270,7 +276,7 @@ __device__ __forceinline__ U settle_order(U b, bool desc) {
 // one warp settles the groups that start in the chunk at c0, in shared memory
 template <int MODE, bool HAS_VAL, typename S, typename U>
 __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, U *key,
-                                         uint32_t *hw, uint32_t *vw, uint32_t *fail) {
+                                         uint32_t *hw, uint32_t *vw, uint32_t *fail, uint32_t fail_bit) {
     constexpr int WORDS = S::kWords;
     const int lane = int(threadIdx.x & 31u);
     const int view = int(n - c0 < uint64_t(S::kView) ? n - c0 : uint64_t(S::kView));
@@ -300,7 +306,7 @@ __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, u
         int e = bit_at_or_above(hw, x + 1, WORDS);
         if (e >= view) {
             if (c0 + uint64_t(view) < n) {                // it runs on past the view
-                if (lane == 0) atomicOr(fail, 1u);
+                if (lane == 0) atomicOr(fail, fail_bit);
                 break;
             }
             e = view;
@@ -325,12 +331,156 @@ __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, u
     __syncwarp();                                         // the warp's shared memory is free again
 }
 
+// one warp settles the groups that start in the chunk at c0 (raising fail_bit in *fail where it cannot)
+template <int MODE, bool HAS_VAL, typename S, typename U>
+__device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, U *key_s,
+                                             uint32_t *hw, uint32_t *vw, uint32_t *fail, uint32_t fail_bit) {
+    constexpr int ITEMS = S::kItems, C = S::kChunk;
+    // v holds the keys as they are where ordering them takes an exclusive-or, else as the sort orders them:
+    // a key that moves is then fetched again from where it came (as a pointer is)
+    constexpr bool RAW = MODE == 0 || MODE == 2, INDEX = HAS_VAL || !RAW;
+    auto ordered = [&](const U &k) { return RAW ? settle_order<MODE>(k, desc) : k; };
+    const int lane = int(threadIdx.x & 31u);
+    const bool full = n - c0 >= uint64_t(32 * ITEMS);
+    const int own = full ? ITEMS : int(n - c0) - lane * ITEMS;      // this lane's keys (may be < 0 or > ITEMS)
+    U v[ITEMS], before{};
+    if (full) {
+        load_run<ITEMS>(v, keys + c0 + lane * ITEMS);
+    } else {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            v[j] = U{};
+            if (j < own) v[j] = keys[c0 + lane * ITEMS + j];
+        }
+    }
+    if (lane == 0 && c0) before = keys[c0 - 1];
+    if constexpr (!RAW) {
+        before = settle_order<MODE>(before, desc);
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) v[j] = settle_order<MODE>(v[j], desc);
+    }
+    // heads and inversions among this lane's keys (bit j: key j)
+    uint32_t hb = 0, vb = 0;
+    {
+        const U up = shfl_up_key(v[ITEMS - 1]);
+        U a = ordered(lane ? up : before);
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const U b = ordered(v[j]);
+            const bool h = !same_masked(a, b, mask);
+            if (h) hb |= 1u << j;
+            else if (key_less(b, a)) vb |= 1u << j;
+            a = b;
+        }
+    }
+    if (c0 == 0 && lane == 0) hb |= 1u;
+    if (!full) hb |= own >= ITEMS ? 0u : own <= 0 ? 0xFFu : 0xFFu << own;     // past the end: each alone
+    vb &= ~hb;
+    const uint32_t heads = __ballot_sync(0xFFFFFFFFu, hb != 0);
+    const bool open = !(heads >> 31) && (heads & 0x7FFFFFFFu) && n - c0 > uint64_t(32 * ITEMS);
+    if (!__any_sync(0xFFFFFFFFu, vb != 0) && !open) return;
+    // this lane's keys of the group that came in, and of the groups that the next chunk settles
+    const uint32_t below = hb ? (hb & (0u - hb)) - 1u : 0xFFu;      // keys before the lane's first head
+    const uint32_t in = (heads & ((1u << lane) - 1u)) == 0 ? below : 0u;
+    const uint32_t out = lane == 31 ? ~below & 0xFFu : 0u;
+    const uint32_t bad_in = vb & in;
+    if (__any_sync(0xFFFFFFFFu, bad_in != 0)) {
+        // settled by the chunk before, if it holds the start and sees the inversion
+        bool lost = bad_in && lane * ITEMS + 31 - __clz(bad_in) >= S::kReach;
+        if (bad_in && c0 > uint64_t(C)) {
+            const U a = settle_order<MODE>(keys[c0 - C - 1], desc), b = settle_order<MODE>(keys[c0 - 1], desc);
+            lost |= same_masked(a, b, mask);
+        }
+        if (lost) atomicOr(fail, fail_bit);
+    }
+    const uint32_t pass = ~hb & ~in & ~out & 0xFFu;          // keys that may pass the one before them
+    bool wide = open;
+    if (!open) {
+        uint32_t moved = 0, from[INDEX ? ITEMS : 1];
+        if constexpr (INDEX) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) from[j] = uint32_t(lane * ITEMS + j);
+        }
+        const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, pass, 1);
+        const bool pass0 = (pass & 1u) && lane, pass8 = lane < 31 && (next & 1u);
+        // one round settles a chunk whose groups have two keys at most
+        const bool several = __any_sync(0xFFFFFFFFu, (pass & (pass << 1)) != 0 || (pass8 && (pass >> (ITEMS - 1))));
+        for (int r = 0;; ++r) {
+            bool swapped = false;
+            // across the lanes: both sides see the same two keys and come to the same answer
+            const U up = shfl_up_key(v[ITEMS - 1]), down = shfl_down_key(v[0]);
+            uint32_t fup = 0, fdown = 0;
+            if constexpr (INDEX) {
+                fup = __shfl_up_sync(0xFFFFFFFFu, from[ITEMS - 1], 1);
+                fdown = __shfl_down_sync(0xFFFFFFFFu, from[0], 1);
+            }
+            if (pass0 && key_less(ordered(v[0]), ordered(up))) {
+                v[0] = up;
+                if constexpr (INDEX) from[0] = fup;
+                moved |= 1u;
+                swapped = true;
+            }
+            if (pass8 && key_less(ordered(down), ordered(v[ITEMS - 1]))) {
+                v[ITEMS - 1] = down;
+                if constexpr (INDEX) from[INDEX ? ITEMS - 1 : 0] = fdown;
+                moved |= 1u << (ITEMS - 1);
+                swapped = true;
+            }
+#pragma unroll
+            for (int j = 1; j < ITEMS; ++j) {
+                if (((pass >> j) & 1u) && key_less(ordered(v[j]), ordered(v[j - 1]))) {
+                    const U t = v[j];
+                    v[j] = v[j - 1];
+                    v[j - 1] = t;
+                    if constexpr (INDEX) {
+                        const uint32_t f = from[INDEX ? j : 0];
+                        from[INDEX ? j : 0] = from[INDEX ? j - 1 : 0];
+                        from[INDEX ? j - 1 : 0] = f;
+                    }
+                    moved |= 3u << (j - 1);
+                    swapped = true;
+                }
+            }
+            if (!several || !__any_sync(0xFFFFFFFFu, swapped)) break;
+            if (r == S::kRounds) {
+                wide = true;
+                break;
+            }
+        }
+        if (!wide) {
+            // every pointer (and key) that moves is read before one is written
+            U *dst = keys + c0 + lane * ITEMS;
+            if constexpr (HAS_VAL) {
+                uint64_t p[ITEMS];
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j)
+                    if ((moved >> j) & 1u) p[j] = vals[c0 + from[j]];
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j)
+                    if ((moved >> j) & 1u) vals[c0 + lane * ITEMS + j] = p[j];
+            }
+            if constexpr (!RAW) {
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j)
+                    if ((moved >> j) & 1u) v[j] = keys[c0 + from[j]];
+                __syncwarp();
+            }
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j)
+                if ((moved >> j) & 1u) dst[j] = v[j];
+        }
+    }
+    if (wide)
+        settle_wide<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc, key_s, hw, vw, fail, fail_bit);
+}
+
 template <typename U, int MODE, bool HAS_VAL>
-__global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HAS_VAL ? 4 : 5) : 6)
+__global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HAS_VAL || (MODE != 0 && MODE != 2) ? 4 : 5) : 6)
     k_settle(Control *__restrict__ ctrl, const SortArrays arrs, uint64_t n, uint32_t desc, unsigned char *status,
              size_t status_bytes, PlanArgs pa) {
     using S = SettleShape<U>;
-    constexpr int THREADS = S::kThreads, ITEMS = S::kItems, C = S::kChunk;
+    constexpr int THREADS = S::kThreads, C = S::kChunk;
     next_may_start();
     after_previous();
     const uint32_t k = ctrl->prefix_passes;
@@ -338,7 +488,7 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
     __shared__ __align__(16) U keys_s[S::kWarps][S::kView];
     __shared__ uint32_t words_s[S::kWarps][2][S::kWords];
     __shared__ uint32_t last;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const PassPlan &end = ctrl->plan[k - 1];
     bool bad = false;
     U *keys = static_cast<U *>(sort_array(arrs, end.dst_keys, HAS_VAL ? kArrKeysA : kArrBuf, &bad));
@@ -356,128 +506,8 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
     for (uint64_t c = uint64_t(blockIdx.x) * S::kWarps + warp; c < chunks; c += stride) {
         // the failure flag is one word for the whole grid: looked at now and then
         if ((++seen & 15u) == 0 && ld_relaxed(&ctrl->settle_fail)) break;
-        const uint64_t c0 = c * C;
-        const bool full = n - c0 >= uint64_t(32 * ITEMS);
-        const int own = full ? ITEMS : int(n - c0) - lane * ITEMS;      // this lane's keys (may be < 0 or > ITEMS)
-        U v[ITEMS], before{};
-        if (full) {
-            load_run<ITEMS>(v, keys + c0 + lane * ITEMS);
-        } else {
-#pragma unroll
-            for (int j = 0; j < ITEMS; ++j) {
-                v[j] = U{};
-                if (j < own) v[j] = keys[c0 + lane * ITEMS + j];
-            }
-        }
-        if (lane == 0 && c0) before = keys[c0 - 1];
-        // heads and inversions among this lane's keys (bit j: key j)
-        uint32_t hb = 0, vb = 0;
-        {
-            const U up = shfl_up_key(v[ITEMS - 1]);
-            U a = settle_order<MODE>(lane ? up : before, desc);
-#pragma unroll
-            for (int j = 0; j < ITEMS; ++j) {
-                const U b = settle_order<MODE>(v[j], desc);
-                const bool h = !same_masked(a, b, mask);
-                if (h) hb |= 1u << j;
-                else if (key_less(b, a)) vb |= 1u << j;
-                a = b;
-            }
-        }
-        if (c0 == 0 && lane == 0) hb |= 1u;
-        if (!full) hb |= own >= ITEMS ? 0u : own <= 0 ? 0xFFu : 0xFFu << own;     // past the end: each alone
-        vb &= ~hb;
-        const uint32_t heads = __ballot_sync(0xFFFFFFFFu, hb != 0);
-        const bool open = !(heads >> 31) && (heads & 0x7FFFFFFFu) && n - c0 > uint64_t(32 * ITEMS);
-        if (!__any_sync(0xFFFFFFFFu, vb != 0) && !open) continue;
-        // this lane's keys of the group that came in, and of the groups that the next chunk settles
-        const uint32_t below = hb ? (hb & (0u - hb)) - 1u : 0xFFu;      // keys before the lane's first head
-        const uint32_t in = (heads & ((1u << lane) - 1u)) == 0 ? below : 0u;
-        const uint32_t out = lane == 31 ? ~below & 0xFFu : 0u;
-        const uint32_t bad_in = vb & in;
-        if (__any_sync(0xFFFFFFFFu, bad_in != 0)) {
-            // settled by the chunk before, if it holds the start and sees the inversion
-            bool lost = bad_in && lane * ITEMS + 31 - __clz(bad_in) >= S::kReach;
-            if (bad_in && c0 > uint64_t(C)) {
-                const U a = settle_order<MODE>(keys[c0 - C - 1], desc), b = settle_order<MODE>(keys[c0 - 1], desc);
-                lost |= same_masked(a, b, mask);
-            }
-            if (lost) atomicOr(&ctrl->settle_fail, 1u);
-        }
-        const uint32_t pass = ~hb & ~in & ~out & 0xFFu;          // keys that may pass the one before them
-        bool wide = open;
-        if (!open) {
-            uint32_t moved = 0, from[HAS_VAL ? ITEMS : 1];
-            if constexpr (HAS_VAL) {
-#pragma unroll
-                for (int j = 0; j < ITEMS; ++j) from[j] = uint32_t(lane * ITEMS + j);
-            }
-            const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, pass, 1);
-            const bool pass0 = (pass & 1u) && lane, pass8 = lane < 31 && (next & 1u);
-            // one round settles a chunk whose groups have two keys at most
-            const bool several = __any_sync(0xFFFFFFFFu, (pass & (pass << 1)) != 0 || (pass8 && (pass >> (ITEMS - 1))));
-            for (int r = 0;; ++r) {
-                bool swapped = false;
-                // across the lanes: both sides see the same two keys and come to the same answer
-                const U up = shfl_up_key(v[ITEMS - 1]), down = shfl_down_key(v[0]);
-                uint32_t fup = 0, fdown = 0;
-                if constexpr (HAS_VAL) {
-                    fup = __shfl_up_sync(0xFFFFFFFFu, from[ITEMS - 1], 1);
-                    fdown = __shfl_down_sync(0xFFFFFFFFu, from[0], 1);
-                }
-                if (pass0 && key_less(settle_order<MODE>(v[0], desc), settle_order<MODE>(up, desc))) {
-                    v[0] = up;
-                    if constexpr (HAS_VAL) from[0] = fup;
-                    moved |= 1u;
-                    swapped = true;
-                }
-                if (pass8 && key_less(settle_order<MODE>(down, desc), settle_order<MODE>(v[ITEMS - 1], desc))) {
-                    v[ITEMS - 1] = down;
-                    if constexpr (HAS_VAL) from[HAS_VAL ? ITEMS - 1 : 0] = fdown;
-                    moved |= 1u << (ITEMS - 1);
-                    swapped = true;
-                }
-#pragma unroll
-                for (int j = 1; j < ITEMS; ++j) {
-                    if (((pass >> j) & 1u) && key_less(settle_order<MODE>(v[j], desc), settle_order<MODE>(v[j - 1], desc))) {
-                        const U t = v[j];
-                        v[j] = v[j - 1];
-                        v[j - 1] = t;
-                        if constexpr (HAS_VAL) {
-                            const uint32_t f = from[HAS_VAL ? j : 0];
-                            from[HAS_VAL ? j : 0] = from[HAS_VAL ? j - 1 : 0];
-                            from[HAS_VAL ? j - 1 : 0] = f;
-                        }
-                        moved |= 3u << (j - 1);
-                        swapped = true;
-                    }
-                }
-                if (!several || !__any_sync(0xFFFFFFFFu, swapped)) break;
-                if (r == S::kRounds) {
-                    wide = true;
-                    break;
-                }
-            }
-            if (!wide) {
-                U *dst = keys + c0 + lane * ITEMS;
-                if constexpr (HAS_VAL) {
-                    uint64_t p[ITEMS];
-#pragma unroll
-                    for (int j = 0; j < ITEMS; ++j)
-                        if ((moved >> j) & 1u) p[j] = vals[c0 + from[j]];
-                    __syncwarp();                    // every pointer that moves has been read
-#pragma unroll
-                    for (int j = 0; j < ITEMS; ++j)
-                        if ((moved >> j) & 1u) vals[c0 + lane * ITEMS + j] = p[j];
-                }
-#pragma unroll
-                for (int j = 0; j < ITEMS; ++j)
-                    if ((moved >> j) & 1u) dst[j] = v[j];
-            }
-        }
-        if (wide)
-            settle_wide<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc != 0, keys_s[warp], words_s[warp][0],
-                                          words_s[warp][1], &ctrl->settle_fail);
+        settle_chunk<MODE, HAS_VAL, S>(keys, vals, c * C, n, mask, desc != 0, keys_s[warp], words_s[warp][0], words_s[warp][1],
+                                       &ctrl->settle_fail, 1u);
     }
     __threadfence();
     __syncthreads();

@@ -1,6 +1,7 @@
 // rsbd8g_seglaunch.cuh - launch sequence of the batched (segmented) sort for one key size:
 //   memset(control, histograms) -> classify -> small-segment block sort -> large-segment
-//   histograms -> per-segment plan -> per pass: memset(look-back words) + segmented onesweep
+//   histograms -> per-segment plan -> per pass: look-back words cleared + segmented onesweep
+//   -> wide keys: settle step, and the passes of the segments it could not settle
 //   -> copy of fully skipped large segments
 // all stream-ordered without host synchronisation, so one CUDA graph can replay a whole batch.
 #pragma once
@@ -11,6 +12,17 @@
 #include "rsbd8g_segmented.cuh"
 
 namespace rsbd8g {
+
+// The launches of wide keys follow one another without draining: a pass that no segment takes costs
+// less (they come in twos and threes).  Keys of up to 4 bytes take every pass, and the CTAs that wait
+// for their turn beside a running pass made a batch of 2^28 uint32 keys 0.4 % slower.
+template <typename U, typename... A>
+cudaError_t seg_launch(void (*kern)(A...), uint32_t grid, int threads, size_t smem, cudaStream_t s,
+                       std::common_type_t<A>... args) {
+    if constexpr (KeyTraits<U>::kDigits >= 8) return launch_after(kern, grid, threads, smem, s, args...);
+    kern<<<grid, threads, smem, s>>>(args...);
+    return cudaGetLastError();
+}
 
 // one-time setup (which also loads the kernel) of the small-segment kernel on device `dev`: its
 // resident CTAs per SM (see SweepKernels in rsbd8g_launch.cuh)
@@ -39,8 +51,7 @@ cudaError_t launch_small_t(const SegArgs &a, const U *in, U *out, cudaStream_t s
     const int occ = small_setup<U, MODE, THREADS, ITEMS>(dev);
     const uint32_t grid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(a.nsegs, uint64_t(occ) * device_sms(dev))));
     LaunchTimer t(s, RSBD8G_KERNEL_SEGMENTED, uint32_t(sizeof(U)), 100, a.nsegs);
-    kern<<<grid, THREADS, SM::kBytes, s>>>(a, in, out);
-    return cudaGetLastError();
+    return seg_launch<U>(kern, grid, THREADS, SM::kBytes, s, a, in, out);
 }
 
 // one-time setup of the segmented scatter kernels (see SweepKernels in rsbd8g_launch.cuh)
@@ -83,7 +94,7 @@ void seg_hist_setup(int dev) {
 
 template <typename U, int MODE, int THREADS, int ITEMS>
 cudaError_t launch_seg_sweeps_t(const SegArgs &a, const SegLayout &L, unsigned char *scratch, const U *in, U *out,
-                                U *buf, uint32_t stall_tile, cudaStream_t s) {
+                                U *buf, uint32_t stall_tile, int phase, cudaStream_t s) {
     // the pipelined pass when the batch has tiles enough to fill it (tiles_max bounds the large tiles)
     using K = SegSweepKernels<U, MODE, THREADS, ITEMS>;
     using SM = typename K::SM;
@@ -103,22 +114,41 @@ cudaError_t launch_seg_sweeps_t(const SegArgs &a, const SegLayout &L, unsigned c
         cudaError_t e;
         {
             LaunchTimer t(s, RSBD8G_KERNEL_MEMSET, uint32_t(sizeof(U)), uint32_t(p), L.tiles_max);
-            e = cudaMemsetAsync(status, 0, L.status_bytes, s);
+            // (wide keys: by a kernel, which knows whether any segment takes the pass)
+            if constexpr (KeyTraits<U>::kDigits >= 8)
+                e = seg_launch<U>(k_seg_clear, uint32_t(device_sms(dev)) * 8, 256, 0, s, a, p, phase, status);
+            else
+                e = cudaMemsetAsync(status, 0, L.status_bytes, s);
         }
         if (e != cudaSuccess) return e;
         LaunchTimer t(s, RSBD8G_KERNEL_SEGMENTED, uint32_t(sizeof(U)), uint32_t(p), L.tiles_max);
         if (pipe)
-            pkern<<<grid, THREADS, PM::kBytes, s>>>(a, p, KeyTraits<U>::kDigits, in, out, buf, status, stall_tile);
+            e = seg_launch<U>(pkern, grid, THREADS, PM::kBytes, s, a, p, phase, KeyTraits<U>::kDigits, in, out, buf, status, stall_tile);
         else
-            kern<<<grid, THREADS, SM::kBytes, s>>>(a, p, KeyTraits<U>::kDigits, in, out, buf, status, stall_tile);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            e = seg_launch<U>(kern, grid, THREADS, SM::kBytes, s, a, p, phase, KeyTraits<U>::kDigits, in, out, buf, status, stall_tile);
+        if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
+// resident CTAs per SM of the segmented settle kernel
 template <typename U, int MODE>
-cudaError_t launch_segmented_mode_t(const Resolved &r, const SegArgs &a, const SegLayout &L, unsigned char *scratch,
+int seg_settle_setup(int dev) {
+    static std::once_flag once[64];
+    static int occ[64];
+    std::call_once(once[dev & 63], [&] {
+        int b = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_seg_settle<U, MODE>, SettleShape<U>::kThreads, 0);
+        occ[dev & 63] = b > 0 ? b : 1;
+    });
+    return occ[dev & 63];
+}
+
+template <typename U, int MODE>
+cudaError_t launch_segmented_mode_t(const Resolved &r, const SegArgs &args, const SegLayout &L, unsigned char *scratch,
                                     const void *in_, void *out_, void *buf_, cudaStream_t s) {
+    SegArgs a = args;
+    a.prefix_ok = KeyTraits<U>::kDigits >= 8 && a.total >= prefix_min_keys(int(sizeof(U))) && !(r.flags & RSBD8G_FLAG_DIAG_STALL);
     const U *in = static_cast<const U *>(in_);
     U *out = static_cast<U *>(out_);
     U *buf = static_cast<U *>(buf_);
@@ -145,27 +175,38 @@ cudaError_t launch_segmented_mode_t(const Resolved &r, const SegArgs &a, const S
         constexpr size_t smem = size_t(hist_lane_copies<P>()) * P * kBuckets * 4;
         auto kern = k_seg_hist<U, MODE, 1024>;
         seg_hist_setup<U, MODE>(dev);
-        kern<<<uint32_t(sms), 1024, smem, s>>>(a, in);
+        e = seg_launch<U>(kern, uint32_t(sms), 1024, smem, s, a, in);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
     {
         LaunchTimer t(s, RSBD8G_KERNEL_PLAN, uint32_t(sizeof(U)), 0, a.nsegs);
         const uint32_t g = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(a.nlarge_max, uint64_t(sms) * 16)));
-        k_seg_plan<<<g, 256, 0, s>>>(a, KeyTraits<U>::kDigits);
+        if constexpr (KeyTraits<U>::kDigits >= 8) e = seg_launch<U>(k_seg_plan_wide<U, MODE>, g, 256, 0, s, a, in);
+        else e = seg_launch<U>(k_seg_plan, g, 256, 0, s, a, KeyTraits<U>::kDigits);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
     constexpr SweepGeometry g0 = seg_sweep_geometry(int(sizeof(U)), 0), g1 = seg_sweep_geometry(int(sizeof(U)), 1);
     const uint32_t stall = (r.flags & RSBD8G_FLAG_DIAG_STALL) ? 1u : 0xFFFFFFFFu;
-    if (L.large_variant == 1 && g1.items != g0.items)
-        e = launch_seg_sweeps_t<U, MODE, g1.threads, g1.items>(a, L, scratch, in, out, buf, stall, s);
-    else
-        e = launch_seg_sweeps_t<U, MODE, g0.threads, g0.items>(a, L, scratch, in, out, buf, stall, s);
-    if (e != cudaSuccess) return e;
+    // wide keys: phase 0 and the settle step, then the passes of the segments that could not be settled
+    for (int phase = 0; phase < (a.prefix_ok ? 2 : 1); ++phase) {
+        if constexpr (KeyTraits<U>::kDigits >= 8) {
+            if (phase) {
+                LaunchTimer t(s, RSBD8G_KERNEL_SETTLE, uint32_t(sizeof(U)), 0, a.nsegs);
+                e = seg_launch<U>(k_seg_settle<U, MODE>, uint32_t(seg_settle_setup<U, MODE>(dev) * sms), SettleShape<U>::kThreads, 0, s, a, out);
+                if (e != cudaSuccess) return e;
+            }
+        }
+        if (L.large_variant == 1 && g1.items != g0.items)
+            e = launch_seg_sweeps_t<U, MODE, g1.threads, g1.items>(a, L, scratch, in, out, buf, stall, phase, s);
+        else
+            e = launch_seg_sweeps_t<U, MODE, g0.threads, g0.items>(a, L, scratch, in, out, buf, stall, phase, s);
+        if (e != cudaSuccess) return e;
+    }
     {
         LaunchTimer t(s, RSBD8G_KERNEL_COPY, uint32_t(sizeof(U)), 0, a.nsegs);
-        k_seg_copy<U><<<uint32_t(sms) * 4, 256, 0, s>>>(a, in, out);
+        e = seg_launch<U>(k_seg_copy<U>, uint32_t(sms) * 4, 256, 0, s, a, in, out, buf);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 template <typename U>
@@ -194,6 +235,11 @@ cudaError_t prepare_segmented_mode_t(int dev) {
     cudaFuncAttributes fa{};
     cudaFuncGetAttributes(&fa, k_seg_classify);
     cudaFuncGetAttributes(&fa, k_seg_plan);
+    cudaFuncGetAttributes(&fa, k_seg_clear);
+    if constexpr (KeyTraits<U>::kDigits >= 8) {
+        cudaFuncGetAttributes(&fa, k_seg_plan_wide<U, MODE>);
+        seg_settle_setup<U, MODE>(dev);
+    }
     cudaFuncGetAttributes(&fa, k_seg_copy<U>);
     return cudaGetLastError();
 }

@@ -25,8 +25,8 @@ struct SegControl {
     uint32_t nsmall;
     uint32_t ntiles;          // tiles of all large segments
     uint32_t small_counter;
-    uint32_t tile_counter[kMaxPasses];
-    uint32_t pad[6];
+    uint32_t tile_counter[2][kMaxPasses];   // by phase (see seg_pass)
+    uint32_t pass_mask[2];    // digits that some segment sorts by, by phase
 };
 
 struct SegArgs {
@@ -43,7 +43,7 @@ struct SegArgs {
     uint32_t *large_tbase;    // [nlarge_max + 1]
     uint32_t *small_seg;      // [nsegs]
     uint32_t *seg_hist;       // [nlarge_max][P][256]: counts, then bucket starts
-    uint32_t *seg_mask;       // [nlarge_max]: surviving digits
+    uint32_t *seg_mask;       // [nlarge_max]: how the segment is sorted (kSegPrefix, kSegFail and below)
     uint32_t *tile_seg;       // [tiles_max]: the large segment (list index) of each tile, by k_seg_hist
     // pointer-table form: segment s lives at ptr_in[s] / ptr_out[s] / ptr_buf[s] (separate arrays;
     // offsets then only give the lengths); null: segment s is at offsets[s] of in / out / buf
@@ -56,6 +56,7 @@ struct SegArgs {
     // above hold for every segment.  rev_ok: the mode honours isrevorder (a uniform property)
     const uint8_t *seg_dir;
     uint32_t rev_ok;
+    uint32_t prefix_ok;       // 8- and 16-byte keys: segments may be sorted by a prefix and settled
 };
 
 // the digit complement (descending sorts) and the effective isrevorder of segment `seg`
@@ -77,6 +78,8 @@ __device__ __forceinline__ U *seg_ptr(const SegArgs &a, const uint64_t *table, c
 // one CTA of 1024 threads classifies every segment; a single 64-bit atomic per warp hands out
 // (list index, tile base) pairs so tile bases grow with the list index
 static __global__ void __launch_bounds__(1024) k_seg_classify(SegArgs a) {
+    next_may_start();
+    after_previous();
     SegControl *c = a.ctrl;
     __shared__ unsigned long long large_ctr;   // (count << 32) | tiles
     __shared__ uint32_t small_ctr;
@@ -146,6 +149,35 @@ static __global__ void __launch_bounds__(1024) k_seg_classify(SegArgs a) {
     }
 }
 
+// How a large segment is sorted: bits 0-15 its surviving digits, bits 16-20 the lowest digit of its
+// prefix, kSegPrefix: by that prefix and the settle step (rsbd8g_prefix.cuh), kSegFail: the settle step
+// found a group too long, so the passes of phase 1 sort the segment by every digit.
+constexpr uint32_t kSegPrefix = 1u << 24, kSegFail = 1u << 25;
+
+// Phase 0 sorts in -> out by the digits of the prefix, or every surviving digit; phase 1 sorts a failed
+// segment from out, by every surviving digit (ending in buf when they are odd in number: k_seg_copy).
+// Is digit `pass` sorted by in `phase`, as the i-th of the segment's k passes?
+template <bool WIDE>
+__device__ __forceinline__ bool seg_pass(uint32_t how, int pass, int phase, int *i, int *k) {
+    uint32_t digits = WIDE ? how & 0xFFFFu : how;
+    if (WIDE && phase) digits = (how & kSegFail) ? digits : 0u;
+    else if (WIDE && (how & kSegPrefix)) digits &= ~((1u << ((how >> 16) & 31u)) - 1u);
+    *k = __popc(digits);
+    *i = __popc(digits & ((1u << pass) - 1u)) + 1;
+    return (digits >> pass) & 1u;
+}
+// the arrays that the i-th of k passes reads and writes
+template <bool WIDE, typename U>
+__device__ __forceinline__ void seg_arrays(int phase, int i, int k, U *in, U *out, U *buf, const void **src, void **dst) {
+    if (WIDE && phase) {
+        *src = (i & 1) ? out : buf;
+        *dst = (i & 1) ? buf : out;
+    } else {
+        *src = (i == 1) ? in : (((k - (i - 1)) % 2 == 0) ? out : buf);
+        *dst = ((k - i) % 2 == 0) ? out : buf;
+    }
+}
+
 // index of the large segment owning global tile gt (tile bases are non-decreasing)
 __device__ __forceinline__ uint32_t seg_of_tile(const uint32_t *tbase, uint32_t nlarge, uint32_t gt) {
     uint32_t lo = 0, hi = nlarge;            // invariant: tbase[lo] <= gt < tbase[hi]
@@ -164,6 +196,8 @@ __global__ void __launch_bounds__(THREADS) k_seg_hist(SegArgs a, const U *__rest
     constexpr int P = KeyTraits<U>::kDigits;
     constexpr int C = hist_lane_copies<P>();
     extern __shared__ __align__(16) uint32_t shl[];   // C lane-class copies, as in k_histogram
+    next_may_start();
+    after_previous();
     const SegControl *c = a.ctrl;
     if (c->abort) return;
     const uint32_t T = c->ntiles, nl = c->nlarge;
@@ -258,11 +292,14 @@ __global__ void __launch_bounds__(THREADS) k_seg_hist(SegArgs a, const U *__rest
 
 // per large segment (one CTA each): bucket starts in place of the counts, surviving-digit mask
 static __global__ void __launch_bounds__(256) k_seg_plan(SegArgs a, int passes) {
-    const SegControl *c = a.ctrl;
+    next_may_start();
+    after_previous();
+    SegControl *c = a.ctrl;
     if (c->abort) return;
     __shared__ uint32_t wsum[8];
     const uint32_t nl = c->nlarge;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    uint32_t all0 = 0;
     for (uint32_t idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         const uint32_t seg = a.large_seg[idx];
         const uint64_t len = seg_len(a.offsets, seg);
@@ -286,55 +323,154 @@ static __global__ void __launch_bounds__(256) k_seg_plan(SegArgs a, int passes) 
             __syncthreads();
         }
         if (t == 0) a.seg_mask[idx] = mask;
+        all0 |= mask;
+    }
+    if (t == 0 && all0) atomicOr(&c->pass_mask[0], all0);
+}
+
+// The plan of 8- and 16-byte keys: beside k_seg_plan's work, samples of the segment decide whether it is
+// sorted by a prefix of its digits (a round of 256 keys for every 2^15 keys, 17 at most: a segment of over
+// 2^20 keys is not sorted by a prefix).  One CTA per segment.
+template <typename U, int MODE>
+__global__ void __launch_bounds__(256) k_seg_plan_wide(SegArgs a, const U *__restrict__ in) {
+    constexpr int P = KeyTraits<U>::kDigits;
+    next_may_start();
+    after_previous();
+    SegControl *c = a.ctrl;
+    if (c->abort) return;
+    __shared__ uint32_t wsum[8], pairs[kMaxPasses];
+    __shared__ __align__(16) U sample[256];
+    const uint32_t nl = c->nlarge;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    uint32_t all0 = 0;
+    for (uint32_t idx = blockIdx.x; idx < nl; idx += gridDim.x) {
+        const uint32_t seg = a.large_seg[idx];
+        const uint64_t len = seg_len(a.offsets, seg);
+        uint32_t mask = 0;
+        for (int p = 0; p < P; ++p) {
+            uint32_t *h = a.seg_hist + (size_t(idx) * P + p) * kBuckets;
+            const uint32_t v = h[t];
+            const int skip = __syncthreads_or(uint64_t(v) == len);
+            uint32_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) wsum[w] = x;
+            __syncthreads();
+            uint32_t before = 0;
+            for (int i = 0; i < w; ++i) before += wsum[i];
+            h[t] = before + x - v;
+            if (!skip) mask |= 1u << p;
+            __syncthreads();
+        }
+        uint32_t how = mask, low = 0;
+        if (a.prefix_ok && __popc(mask) > 3) {
+            const U *src = seg_ptr(a, a.ptr_in, in, seg);
+            const uint64_t r = (len >> 15) + 1u;       // (a round's pairs, 32,640, are for as many keys)
+            const uint32_t rounds = r > 17 ? 17u : uint32_t(r);
+            prefix_sample<U, 256>(sample, len, rounds, uint64_t(idx) * 17u, pairs, [&](uint64_t i) { return filter_key<MODE>(src[i]); });
+            if (prefix_choose(pairs, mask, len, uint64_t(rounds) * 256u * 255u / 2u, &low)) how |= kSegPrefix | (low << 16);
+            __syncthreads();
+        }
+        if (t == 0) a.seg_mask[idx] = how;
+        all0 |= (how & kSegPrefix) ? mask & ~((1u << low) - 1u) : mask;
+    }
+    if (t == 0 && all0) atomicOr(&c->pass_mask[0], all0);
+}
+
+// the look-back words of all tiles cleared for pass `pass` of `phase`, if any segment takes it
+static __global__ void __launch_bounds__(256) k_seg_clear(SegArgs a, int pass, int phase, uint32_t *__restrict__ status) {
+    next_may_start();
+    after_previous();
+    const SegControl *c = a.ctrl;
+    if (c->abort || !((c->pass_mask[phase] >> pass) & 1u)) return;
+    const uint64_t words = uint64_t(c->ntiles) * (kBuckets / 4);
+    for (uint64_t i = uint64_t(blockIdx.x) * 256u + threadIdx.x; i < words; i += uint64_t(gridDim.x) * 256u)
+        reinterpret_cast<uint4 *>(status)[i] = make_uint4(0, 0, 0, 0);
+}
+
+// the settle step of the segments sorted by a prefix, in place in their output: warps take quarters of
+// the large segments' tiles in turn (a quarter: the chunks that start in it)
+template <typename U, int MODE>
+__global__ void __launch_bounds__(SettleShape<U>::kThreads, 4) k_seg_settle(SegArgs a, U *__restrict__ out) {
+    using S = SettleShape<U>;
+    next_may_start();
+    after_previous();
+    SegControl *c = a.ctrl;
+    if (c->abort) return;
+    __shared__ __align__(16) U keys_s[S::kWarps][S::kView];
+    __shared__ uint32_t words_s[S::kWarps][2][S::kWords];
+    const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
+    const uint64_t units = uint64_t(c->ntiles) * 4u, stride = uint64_t(gridDim.x) * S::kWarps;
+    const uint32_t part = a.tile / 4u;
+    for (uint64_t u = uint64_t(blockIdx.x) * S::kWarps + warp; u < units; u += stride) {
+        const uint32_t gt = uint32_t(u / 4u), idx = a.tile_seg[gt], how = a.seg_mask[idx];
+        if (!(how & kSegPrefix)) continue;
+        const uint32_t seg = a.large_seg[idx];
+        const uint64_t n = seg_len(a.offsets, seg);
+        const uint64_t k0 = uint64_t(gt - a.large_tbase[idx]) * a.tile + uint64_t(u % 4u) * part;
+        if (k0 >= n) continue;
+        const uint64_t k1 = k0 + part < n ? k0 + part : n;
+        U *keys = seg_ptr(a, a.ptr_out, out, seg);
+        const U mask = prefix_mask<U>((how >> 16) & 31u);
+        const bool desc = seg_dmask(a, seg) != 0;
+        for (uint64_t x = (k0 + S::kChunk - 1) / S::kChunk; x * S::kChunk < k1; ++x)
+            settle_chunk<MODE, false, S>(keys, static_cast<uint64_t *>(nullptr), x * S::kChunk, n, mask, desc, keys_s[warp],
+                                         words_s[warp][0], words_s[warp][1], a.seg_mask + idx, kSegFail);
+        __syncwarp();
+        if (lane == 0 && (ld_relaxed(a.seg_mask + idx) & kSegFail)) atomicOr(&c->pass_mask[1], how & 0xFFFFu);
     }
 }
 
 // one onesweep pass over the tiles of every large segment
 template <typename U, int MODE, int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS, onesweep_min_blocks<U, false, THREADS>())
-    k_seg_sweep(SegArgs a, int pass, int passes, const U *__restrict__ in, U *__restrict__ out,
+    k_seg_sweep(SegArgs a, int pass, int phase, int passes, const U *__restrict__ in, U *__restrict__ out,
                 U *__restrict__ buf, uint32_t *__restrict__ status, uint32_t stall_tile) {
     using L = OnesweepSmem<U, false, THREADS, ITEMS>;
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long *bstart = reinterpret_cast<unsigned long long *>(smem + L::kOffBstart);
     uint32_t *misc = reinterpret_cast<uint32_t *>(smem + L::kOffMisc);
+    after_previous();
     SegControl *c = a.ctrl;
-    if (c->abort) return;
+    if (c->abort || !((c->pass_mask[phase] >> pass) & 1u)) return;
     const uint32_t T = c->ntiles;
     const uint64_t spin_limit = a.spin_limit_ns;
     sweep_init_smem<U, MODE, false, THREADS, ITEMS, uint32_t>(smem);
     for (;;) {
         if (threadIdx.x == 0) {
-            misc[0] = atomicAdd(&c->tile_counter[pass], 1u);
+            misc[0] = atomicAdd(&c->tile_counter[phase][pass], 1u);
             misc[1] = 0;
         }
         __syncthreads();
         const uint32_t gt = misc[0];
         if (gt >= T) break;
         const uint32_t idx = a.tile_seg[gt];
-        const uint32_t mask = a.seg_mask[idx];
-        if (!((mask >> pass) & 1u)) {        // this digit is skipped for the segment
+        int i, k;
+        if (!seg_pass<KeyTraits<U>::kDigits >= 8>(a.seg_mask[idx], pass, phase, &i, &k)) {        // this digit is skipped for the segment
             __syncthreads();
             continue;
         }
         const uint32_t seg = a.large_seg[idx];
         const uint64_t len = seg_len(a.offsets, seg);
-        const int k = __popc(mask), i = __popc(mask & ((1u << pass) - 1u)) + 1;
         U *sin = seg_ptr(a, a.ptr_in, in, seg), *sout = seg_ptr(a, a.ptr_out, out, seg);
         U *sbuf = seg_ptr(a, a.ptr_buf, buf, seg);
-        const U *src = (i == 1) ? sin : (((k - (i - 1)) % 2 == 0) ? sout : sbuf);
-        U *dst = ((k - i) % 2 == 0) ? sout : sbuf;
+        const void *src;
+        void *dst;
+        seg_arrays<KeyTraits<U>::kDigits >= 8>(phase, i, k, sin, sout, sbuf, &src, &dst);
         const uint32_t *bs = a.seg_hist + (size_t(idx) * passes + pass) * kBuckets;
         for (int j = threadIdx.x; j < kBuckets; j += THREADS) bstart[j] = bs[j];
         SweepTile<U, uint32_t> t;
-        t.src_k = src;
-        t.dst_k = dst;
+        t.src_k = static_cast<const U *>(src);
+        t.dst_k = static_cast<U *>(dst);
         t.src_v = nullptr;
         t.dst_v = nullptr;
         t.status = status + size_t(a.large_tbase[idx]) * kBuckets;
         t.n = len;
         t.tile = gt - a.large_tbase[idx];
-        t.reverse = seg_rev(a, seg) && i == 1;
+        t.reverse = seg_rev(a, seg) && i == 1 && phase == 0;
         sweep_tile<U, MODE, false, THREADS, ITEMS, uint32_t>(smem, t, bstart, pass, seg_dmask(a, seg), &c->error, &c->abort,
                                                              spin_limit, stall_tile);
     }
@@ -357,30 +493,31 @@ struct SegPipeTile {
 };
 
 template <typename U>
-__device__ __forceinline__ bool seg_pipe_tile(const SegArgs &a, int pass, int passes, const U *in, U *out, U *buf,
+__device__ __forceinline__ bool seg_pipe_tile(const SegArgs &a, int pass, int phase, int passes, const U *in, U *out, U *buf,
                                               uint32_t *status, uint32_t gt, SegPipeTile &t) {
     const uint32_t idx = a.tile_seg[gt];
-    const uint32_t mask = a.seg_mask[idx];
+    int i, k;
     t.src = nullptr;
-    if (!((mask >> pass) & 1u)) return false;          // this digit is skipped for the segment
+    if (!seg_pass<KeyTraits<U>::kDigits >= 8>(a.seg_mask[idx], pass, phase, &i, &k)) {       // this digit is skipped for the segment
+        atomicMax(&a.ctrl->tile_counter[phase][pass], a.large_tbase[idx + 1]);     // and for its tiles still unclaimed
+        return false;
+    }
     const uint32_t seg = a.large_seg[idx];
-    const int k = __popc(mask), i = __popc(mask & ((1u << pass) - 1u)) + 1;
     U *sin = seg_ptr(a, a.ptr_in, in, seg), *sout = seg_ptr(a, a.ptr_out, out, seg);
     U *sbuf = seg_ptr(a, a.ptr_buf, buf, seg);
-    t.src = (i == 1) ? sin : (((k - (i - 1)) % 2 == 0) ? sout : sbuf);
-    t.dst = ((k - i) % 2 == 0) ? sout : sbuf;
+    seg_arrays<KeyTraits<U>::kDigits >= 8>(phase, i, k, sin, sout, sbuf, &t.src, &t.dst);
     t.bs = a.seg_hist + (size_t(idx) * passes + pass) * kBuckets;
     t.status = status + size_t(a.large_tbase[idx]) * kBuckets;
     t.n = seg_len(a.offsets, seg);
     t.tile = gt - a.large_tbase[idx];
-    t.reverse = (seg_rev(a, seg) && i == 1) ? 1u : 0u;
+    t.reverse = (seg_rev(a, seg) && i == 1 && phase == 0) ? 1u : 0u;
     t.dmask = seg_dmask(a, seg);
     return true;
 }
 
 template <typename U, int MODE, int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS, 2)
-    k_seg_sweep_pipe(SegArgs a, int pass, int passes, const U *__restrict__ in, U *__restrict__ out,
+    k_seg_sweep_pipe(SegArgs a, int pass, int phase, int passes, const U *__restrict__ in, U *__restrict__ out,
                      U *__restrict__ buf, uint32_t *__restrict__ status, uint32_t stall_tile) {
     static_assert(THREADS == 2 * kBuckets, "threads 0..255 scan, threads 256..511 look back");
     using L = PipeSmem<U, THREADS, ITEMS>;
@@ -394,8 +531,9 @@ __global__ void __launch_bounds__(THREADS, 2)
     uint32_t *tsall = reinterpret_cast<uint32_t *>(smem + L::kOffTs);
     uint32_t *cntall = reinterpret_cast<uint32_t *>(smem + L::kOffCnt);
     uint32_t *misc = reinterpret_cast<uint32_t *>(smem + L::kOffMisc);   // [0] next tile [1] bad [2..9] scan
+    after_previous();
     SegControl *c = a.ctrl;
-    if (c->abort) return;
+    if (c->abort || !((c->pass_mask[phase] >> pass) & 1u)) return;
     // the descriptors of the claimed tiles, two slots used in turn: thread 0 looks a tile up once
     // when it claims it and the CTA reads the descriptor from here one iteration later
     static_assert(2 * sizeof(SegPipeTile) <= 128, "descriptor slots fit the auxiliary area");
@@ -410,10 +548,10 @@ __global__ void __launch_bounds__(THREADS, 2)
 
     for (int i = tid; i < R::kWords; i += THREADS) utab[i] = 0u;
     if (tid == 0) {
-        const uint32_t g = atomicAdd(&c->tile_counter[pass], 1u);
+        const uint32_t g = atomicAdd(&c->tile_counter[phase][pass], 1u);
         misc[0] = g;
         misc[1] = 0u;
-        if (g < T) seg_pipe_tile<U>(a, pass, passes, in, out, buf, status, g, slots[0]);
+        if (g < T) seg_pipe_tile<U>(a, pass, phase, passes, in, out, buf, status, g, slots[0]);
     }
     __syncthreads();
     uint32_t gtB = misc[0];
@@ -423,6 +561,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     int par = 0;
     for (uint32_t it = 0;; ++it) {
         const bool claimed = gtB < T;
+        if (!claimed) next_may_start();          // the last of this CTA's tiles
         if (!hasA && !claimed) break;
         if (claimed) B = slots[it & 1u];
         const bool hasB = claimed && B.src != nullptr;
@@ -430,9 +569,9 @@ __global__ void __launch_bounds__(THREADS, 2)
         uint32_t *cntB = cntall + par * kBuckets, *cntA = cntall + (par ^ 1) * kBuckets;
         uint32_t next = 0xFFFFFFFFu;
         if (claimed && tid == 0) {
-            next = atomicAdd(&c->tile_counter[pass], 1u);   // the tile after B: its keys go to L2 now
+            next = atomicAdd(&c->tile_counter[phase][pass], 1u);   // the tile after B: its keys go to L2 now
             SegPipeTile &N = slots[(it & 1u) ^ 1u];
-            if (next < T && seg_pipe_tile<U>(a, pass, passes, in, out, buf, status, next, N) && a.prefetch)
+            if (next < T && seg_pipe_tile<U>(a, pass, phase, passes, in, out, buf, status, next, N) && a.prefetch)
                 prefetch_tile<TILE>(static_cast<const U *>(N.src), N.n, N.tile, N.reverse != 0);
         }
         // the look-back threads load A's first window now: the loads complete while B is ranked
@@ -532,20 +671,26 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
 }
 
-// large segments with every digit skipped: plain or reversed copy (one warp per segment)
+// large segments with every digit skipped: plain or reversed copy; and the failed ones whose passes ended
+// in buf (one warp per segment)
 template <typename U>
-__global__ void __launch_bounds__(256) k_seg_copy(SegArgs a, const U *__restrict__ in, U *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_seg_copy(SegArgs a, const U *__restrict__ in, U *__restrict__ out,
+                                                  const U *__restrict__ buf) {
+    next_may_start();
+    after_previous();
     const SegControl *c = a.ctrl;
     if (c->abort) return;
     const uint32_t nl = c->nlarge;
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; idx < nl; idx += (gridDim.x * blockDim.x) >> 5) {
-        if (a.seg_mask[idx]) continue;
+        const uint32_t how = a.seg_mask[idx];
+        const bool back = (how & kSegFail) && (__popc(how & 0xFFFFu) & 1);
+        if ((how & 0xFFFFu) && !back) continue;
         const uint32_t seg = a.large_seg[idx];
         const uint64_t len = seg_len(a.offsets, seg);
-        const U *src = seg_ptr(a, a.ptr_in, in, seg);
+        const U *src = back ? seg_ptr(a, a.ptr_buf, buf, seg) : seg_ptr(a, a.ptr_in, in, seg);
         U *dst = seg_ptr(a, a.ptr_out, out, seg);
-        const bool rev = seg_rev(a, seg);
+        const bool rev = seg_rev(a, seg) && !back;
         for (uint64_t i = lane; i < len; i += 32) dst[i] = src[rev ? len - 1 - i : i];
     }
 }
@@ -579,6 +724,8 @@ __global__ void __launch_bounds__(THREADS) k_seg_small(SegArgs a, const U *__res
     uint32_t *wofs = reinterpret_cast<uint32_t *>(smem + L::kOffWofs);
     uint32_t *wmaskall = reinterpret_cast<uint32_t *>(smem + L::kOffWmask);
     uint32_t *misc = reinterpret_cast<uint32_t *>(smem + L::kOffMisc);   // [0] job [1] skip [2..9] scan
+    next_may_start();
+    after_previous();
     SegControl *c = a.ctrl;
     if (c->abort) return;
     const uint32_t ns = c->nsmall;

@@ -109,3 +109,38 @@ def test_prefix_sort_of_16_byte_keys(kind, case):
     assert rs.radixsortcopy(x, y, "dscfwdorder", "native", key_dtype=kind)
     want = O.sortcopy_wide(w, kind, "native", "dscfwdorder")
     assert np.array_equal(y.cpu().numpy().view(np.uint64).reshape(n, 2), np.asarray(want).reshape(n, 2))
+
+
+@pytest.mark.parametrize("kind", ["i64", "f64", "u128"])
+def test_prefix_in_batches(kind):
+    """the segmented sort decides per segment: uniform segments, clusters that are settled or bring the
+    plain passes back (an even and an odd number of digits), long runs of equal keys, few digits"""
+    import torch
+    from radixsortbidi8_gb300 import api, batched
+    segs = []
+    for i, n in enumerate([6145, 262144, 7001, 50, 100003, 248 * 40, 8192 * 3 + 1, 200000, 1 << 19, 150000, 99999]):
+        for j, case in enumerate(["uniform", "pairs", "groups_of_5", "cluster_480", "few_values"]):
+            if (i + j) % 2:
+                segs.append(CASES[case](max(n, 600) if case.startswith("cluster") else n))
+        segs.append(with_cluster(max(n, 6000), 500, 3) & np.uint64((1 << 56) - 1))      # seven digits
+        segs.append(with_cluster(max(n, 6000), 520, 5000))
+    a = np.concatenate(segs)
+    offs = np.zeros(len(segs) + 1, dtype=np.int64)
+    np.cumsum([s.size for s in segs], out=offs[1:])
+    if kind == "u128":
+        w = np.stack([S.uniform_bits(4, a.size, np.uint64), a], axis=1)
+        x, kt = torch.from_numpy(w.view(np.int64).reshape(-1)).cuda(), "u128"
+    else:
+        kt = np.int64 if kind == "i64" else np.float64
+        x = torch.from_numpy(a.view(np.int64)).cuda()
+    s = batched.SegmentedSorter(x, torch.from_numpy(offs).cuda(), "dscfwdorder", "native", key_dtype=kt)
+    for out in (s.run(), s.capture().replay()):
+        torch.cuda.synchronize()
+        assert s.status() == api.OK
+        got = out.cpu().numpy()
+        for b, e in zip(offs[:-1], offs[1:]):
+            if kind == "u128":
+                want = O.sortcopy_wide(w[b:e], "u128", "native", "dscfwdorder")
+                assert np.array_equal(got[2 * b:2 * e].view(np.uint64).reshape(-1, 2), np.asarray(want).reshape(-1, 2))
+            else:
+                assert same_bits(got[b:e].view(kt), O.sortcopy(a[b:e].view(kt), "native", "dscfwdorder"))
