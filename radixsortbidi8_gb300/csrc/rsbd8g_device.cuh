@@ -143,6 +143,15 @@ __device__ __forceinline__ uint32_t digit_of(U k, int pass) {
     return uint32_t(k >> (pass * kRadixBits)) & (kBuckets - 1);
 }
 
+// (digit `pass` of the filtered key k, complemented by dmask) << LOG: a digit as a byte offset into a
+// table, by one rotation and one mask
+template <int LOG, typename U>
+__device__ __forceinline__ uint32_t digit_scaled(U k, int pass, uint32_t dmask) {
+    uint32_t w = uint32_t(k);
+    if constexpr (sizeof(U) == 8) w = pass < 4 ? w : uint32_t(k >> 32);
+    return (__funnelshift_r(w, w, uint32_t(pass * kRadixBits - LOG)) & ((kBuckets - 1u) << LOG)) ^ (dmask << LOG);
+}
+
 // ---- wide keys --------------------------------------------------------------------------
 // Two little-endian 64-bit words in 16-byte storage, as the reference's test128 / longdoubletest128
 // (Radixsortbidi8.hpp:1061-1100, :1969-2404).  KeyWide<64>: a 128-bit key (integer, or a float
@@ -178,6 +187,11 @@ __host__ __device__ __forceinline__ KeyWide<HB> key_not(KeyWide<HB> k) {
 template <int HB>
 __device__ __forceinline__ uint32_t digit_of(KeyWide<HB> k, int pass) {
     return uint32_t(pass < 8 ? (k.lo >> (pass * kRadixBits)) : (k.hi >> ((pass - 8) * kRadixBits))) & (kBuckets - 1);
+}
+
+template <int LOG, int HB>
+__device__ __forceinline__ uint32_t digit_scaled(KeyWide<HB> k, int pass, uint32_t dmask) {
+    return digit_scaled<LOG>(pass < 8 ? k.lo : k.hi, pass & 7, dmask);
 }
 
 // K(b) of the same 8 filter combinations on the (64 + HB)-bit key; the result keeps `hi` within

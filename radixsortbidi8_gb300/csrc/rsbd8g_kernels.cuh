@@ -391,6 +391,8 @@ __device__ __forceinline__ uint32_t pass_digit(U k, int pass, uint32_t dmask) {
 // leader advances the count with one returning atomic, clears the mask and hands the old count to
 // its peers with a shuffle: four operations and a shuffle per key, but half as many units to scan
 // per tile, which pays for small tiles.
+//   The words of a warp's two half-warp units lie side by side, (digit, unit) at 2 * digit + unit: each unit's
+// lanes keep to their own 16 banks, and the scans over the units take both words at a time.
 // Both tables take (THREADS / 16) * 256 words.  A unit holds at most LANES * ITEMS keys, so counts
 // stay below 2^16.  Large tiles keep their ranks packed in registers and recompute the digit when the
 // key is staged (registers are what limits them); small tiles keep (rank << 8) | digit per key.
@@ -401,9 +403,11 @@ __device__ __forceinline__ uint32_t pass_digit(U k, int pass, uint32_t dmask) {
 // first lane stores the count into the table word afterwards, where the scan finds it: the ranks
 // are the ones the table would have given.
 
-template <int MODE, typename U>
+// a key's digit << LOG; FULL: the tile has no padding slots
+template <int MODE, int LOG, bool FULL, typename U>
 __device__ __forceinline__ uint32_t slot_digit(const U &k, uint32_t slot, uint32_t tvalid, int pass, uint32_t dmask) {
-    return slot < tvalid ? pass_digit<MODE>(k, pass, dmask) : uint32_t(kBuckets - 1);   // padding ranks last
+    const uint32_t d = digit_scaled<LOG>(filter_key<MODE>(k), pass, dmask);
+    return FULL || slot < tvalid ? d : uint32_t(kBuckets - 1) << LOG;   // padding ranks last
 }
 
 // the unit size that measured faster for a tile of THREADS * ITEMS keys
@@ -430,13 +434,24 @@ struct TileRank {
     static constexpr int kRankRegs = kPacked ? (ITEMS + kPerReg - 1) / kPerReg : ITEMS;
 
     __device__ static uint32_t slot0() { return (threadIdx.x / LANES) * LANES * ITEMS + threadIdx.x % LANES; }
-    // the unit's count (later offset) words
-    __device__ static uint32_t *row(uint32_t *tab) { return tab + (threadIdx.x / LANES) * kBuckets; }
+    // words from one digit's to the next, and the byte offset of a digit's word as a shift of the digit
+    static constexpr int kStep = 32 / LANES;
+    static constexpr int kLog = LANES == 16 ? 3 : 2;
+    // the unit's count (later offset) words: digit d's is row(tab)[d * kStep]
+    __device__ static uint32_t *row(uint32_t *tab) {
+        return tab + (threadIdx.x / 32) * kStep * kBuckets + (LANES == 16 ? (threadIdx.x / 16) % 2 : 0);
+    }
+    __device__ static uint32_t *word(uint32_t *row, uint32_t scaled) {
+        return reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(row) + scaled);
+    }
+    __device__ static const uint32_t *word(const uint32_t *row, uint32_t scaled) {
+        return reinterpret_cast<const uint32_t *>(reinterpret_cast<const unsigned char *>(row) + scaled);
+    }
 
     // rank this lane's ITEMS keys within its unit (the unit's masks clear, its counts zero); with
     // HOT > 0 the digits in `hot` ((digit1 << 16) | digit0, kNoHot for none) are ranked by ballots
     // (PADS false: padding slots are left out of the table, and get no rank)
-    template <int MODE, int HOT = 0, bool PADS = true, typename U>
+    template <int MODE, int HOT = 0, bool PADS = true, bool FULL = false, typename U>
     __device__ static void rank(const U (&keys)[ITEMS], uint32_t (&rk)[kRankRegs], uint32_t *tab, uint32_t slot0,
                                 uint32_t tvalid, int pass, uint32_t dmask, uint32_t hot = kNoHotPair) {
         uint32_t *crow = row(tab);
@@ -444,11 +459,11 @@ struct TileRank {
         // this unit's lanes within a warp ballot
         const uint32_t ushift = LANES == 16 ? (threadIdx.x & 16u) : 0u;
         const uint32_t umask = LANES == 16 ? 0xFFFFu : 0xFFFFFFFFu;
-        const uint32_t h0 = hot & 0xFFFFu, h1 = hot >> 16;
+        const uint32_t h0 = (hot & 0xFFFFu) << kLog, h1 = (hot >> 16) << kLog;
         uint32_t hc0 = 0, hc1 = 0;          // the unit's running counts of the hot digits
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
-            const uint32_t d = slot_digit<MODE>(keys[i], slot0 + uint32_t(LANES) * i, tvalid, pass, dmask);
+            const uint32_t d = slot_digit<MODE, kLog, FULL>(keys[i], slot0 + uint32_t(LANES) * i, tvalid, pass, dmask);
             bool is_hot = !PADS && slot0 + uint32_t(LANES) * i >= tvalid;
             uint32_t rh = 0;
             if constexpr (HOT > 0) {
@@ -469,76 +484,83 @@ struct TileRank {
             }
             uint32_t r;
             if constexpr (LANES == 16) {
-                if (!is_hot) atomicOr(crow + d, bit);
+                uint32_t *cw = word(crow, d);
+                if (!is_hot) atomicOr(cw, bit);
                 __syncwarp();
-                const uint32_t w = is_hot ? 0u : crow[d];
+                const uint32_t w = is_hot ? 0u : *cw;
                 __syncwarp();
                 const uint32_t peers = w & 0xFFFFu;
                 const uint32_t lower = uint32_t(__popc(peers & below));
                 if (!is_hot && lower == 0) {
-                    if constexpr (DENSE) crow[d] = ((w >> 16) + uint32_t(__popc(peers))) << 16;
-                    else atomicAdd(crow + d, (uint32_t(__popc(peers)) << 16) - peers);
+                    if constexpr (DENSE) *cw = ((w >> 16) + uint32_t(__popc(peers))) << 16;
+                    else atomicAdd(cw, (uint32_t(__popc(peers)) << 16) - peers);
                 }
                 __syncwarp();      // the cleared mask is visible to the next item's updates
                 r = is_hot ? rh : (w >> 16) + lower;
             } else {
                 uint32_t *mrow = tab + (THREADS / 32) * kBuckets + (threadIdx.x / 32) * kBuckets;
-                if (!is_hot) atomicOr(mrow + d, bit);
+                uint32_t *mw = word(mrow, d);
+                if (!is_hot) atomicOr(mw, bit);
                 __syncwarp();
-                const uint32_t peers = is_hot ? 0u : mrow[d];
+                const uint32_t peers = is_hot ? 0u : *mw;
                 __syncwarp();
                 const uint32_t lower = uint32_t(__popc(peers & below));
                 uint32_t before = 0;
                 if (!is_hot && lower == 0) {
-                    before = atomicAdd(crow + d, uint32_t(__popc(peers)));
-                    mrow[d] = 0u;
+                    before = atomicAdd(word(crow, d), uint32_t(__popc(peers)));
+                    *mw = 0u;
                 }
                 __syncwarp();
                 const uint32_t src = peers ? uint32_t(__ffs(peers) - 1) : 0u;
                 const uint32_t b = __shfl_sync(0xFFFFFFFFu, before, src);
                 r = is_hot ? rh : b + lower;
             }
-            if constexpr (!kPacked) rk[i] = (r << 8) | d;
+            if constexpr (!kPacked) rk[i] = (r << 16) | d;      // (a scaled digit is below 2^11)
             else if (i % kPerReg != 0) rk[i / kPerReg] |= r << (kRankBits * (i % kPerReg));
             else rk[i / kPerReg] = r;
         }
         if constexpr (HOT > 0) {
             // the hot digits' unit counts go where the table keeps counts (their words are zero)
             if (threadIdx.x % LANES == 0) {
-                if (h0 < kBuckets) crow[h0] = hc0 << kShift;
-                if (HOT > 1 && h1 < kBuckets) crow[h1] = hc1 << kShift;
+                if (h0 < (uint32_t(kBuckets) << kLog)) *word(crow, h0) = hc0 << kShift;
+                if (HOT > 1 && h1 < (uint32_t(kBuckets) << kLog)) *word(crow, h1) = hc1 << kShift;
             }
         }
     }
 
     __device__ static uint32_t rank_of(const uint32_t (&rk)[kRankRegs], int i) {
-        if constexpr (!kPacked) return rk[i] >> 8;
+        if constexpr (!kPacked) return rk[i] >> 16;
         else return (rk[i / kPerReg] >> (kRankBits * (i % kPerReg))) & ((1u << kRankBits) - 1u);
     }
 
-    // the digit item i was ranked under (slot = its slot in the tile)
-    template <int MODE, typename U>
+    // the digit item i was ranked under (slot = its slot in the tile), scaled as word() takes it
+    template <int MODE, bool FULL = false, typename U>
     __device__ static uint32_t digit_of_item(const uint32_t (&rk)[kRankRegs], int i, const U &k, uint32_t slot,
                                              uint32_t tvalid, int pass, uint32_t dmask) {
-        if constexpr (!kPacked) return rk[i] & 0xFFu;
-        else return slot_digit<MODE>(k, slot, tvalid, pass, dmask);
+        if constexpr (!kPacked) return rk[i] & 0xFFFFu;
+        else return slot_digit<MODE, kLog, FULL>(k, slot, tvalid, pass, dmask);
     }
 
     // digit d's count in the tile: the sum over the units
-    __device__ static uint32_t total(const uint32_t *tab, int d) {
-        uint32_t run = 0;
-#pragma unroll
-        for (int u = 0; u < kUnits; ++u) run += tab[u * kBuckets + d] >> kShift;
-        return run;
-    }
+    __device__ static uint32_t total(const uint32_t *tab, int d) { return total_of<0, kUnits>(tab, d); }
 
-    // digit d's count over the units [U0, U1)
+    // digit d's count over the units [U0, U1) (half-warp units: both of a warp at a time; the words' counts
+    // are summed where they lie, as a tile holds fewer than 2^16 keys)
     template <int U0, int U1>
     __device__ static uint32_t total_of(const uint32_t *tab, int d) {
         uint32_t run = 0;
+        if constexpr (LANES == 16) {
+            static_assert(U0 % 2 == 0 && U1 % 2 == 0, "whole warps");
 #pragma unroll
-        for (int u = U0; u < U1; ++u) run += tab[u * kBuckets + d] >> kShift;
-        return run;
+            for (int u = U0; u < U1; u += 2) {
+                const uint2 v = *reinterpret_cast<const uint2 *>(tab + u * kBuckets + 2 * d);
+                run += v.x + v.y;
+            }
+        } else {
+#pragma unroll
+            for (int u = U0; u < U1; ++u) run += tab[u * kBuckets + d];
+        }
+        return run >> kShift;
     }
 
     // replace digit d's unit counts by the units' staging offsets, the first one at the tile start ts
@@ -547,11 +569,22 @@ struct TileRank {
     // the same for the units [U0, U1), the first of them starting at ts
     template <int U0, int U1>
     __device__ static void offsets_of(uint32_t *tab, int d, uint32_t ts) {
+        if constexpr (LANES == 16) {
 #pragma unroll
-        for (int u = U0; u < U1; ++u) {
-            const uint32_t c = tab[u * kBuckets + d] >> kShift;
-            tab[u * kBuckets + d] = ts;
-            ts += c;
+            for (int u = U0; u < U1; u += 2) {
+                uint2 *p = reinterpret_cast<uint2 *>(tab + u * kBuckets + 2 * d);
+                const uint2 c = *p;
+                const uint32_t mid = ts + (c.x >> kShift);
+                *p = make_uint2(ts, mid);
+                ts = mid + (c.y >> kShift);
+            }
+        } else {
+#pragma unroll
+            for (int u = U0; u < U1; ++u) {
+                const uint32_t c = tab[u * kBuckets + d];
+                tab[u * kBuckets + d] = ts;
+                ts += c;
+            }
         }
     }
 
@@ -561,7 +594,8 @@ struct TileRank {
         uint32_t *rows = tab + (threadIdx.x / 32) * (32 / LANES) * kBuckets;
         __syncwarp();
 #pragma unroll
-        for (int i = threadIdx.x % 32; i < (32 / LANES) * kBuckets; i += 32) rows[i] = 0u;
+        for (int i = threadIdx.x % 32; i < (32 / LANES) * kBuckets / 4; i += 32)
+            reinterpret_cast<uint4 *>(rows)[i] = make_uint4(0, 0, 0, 0);
     }
 };
 
@@ -667,6 +701,16 @@ __device__ __forceinline__ bool lookback_walk(const S *status, uint32_t tile, in
 // 30-bit look-back words (sorts of fewer than 2^30 keys), 64-bit beyond
 template <typename S>
 using TileOffset = std::conditional_t<std::is_same_v<S, uint32_t>, int32_t, long long>;
+// is output position g inside an array of n elements (a negative g is not)
+__device__ __forceinline__ bool inside(int32_t g, uint64_t n) { return uint32_t(g) < uint32_t(n); }   // n < 2^30
+__device__ __forceinline__ bool inside(long long g, uint64_t n) { return uint64_t(g) < n; }
+
+// the entry of a staged key's digit in the tile's offset table
+template <int MODE, typename G, typename U>
+__device__ __forceinline__ const G *tile_offset(const G *gofs, const U &k, int pass, uint32_t dmask) {
+    return reinterpret_cast<const G *>(reinterpret_cast<const unsigned char *>(gofs) +
+                                       digit_scaled<sizeof(G) == 4 ? 2 : 3>(filter_key<MODE>(k), pass, dmask));
+}
 
 template <typename U, bool HAS_VAL, int THREADS>
 constexpr int onesweep_min_blocks() {
@@ -766,7 +810,7 @@ __device__ __forceinline__ void sweep_tile(unsigned char *smem, const SweepTile<
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const uint32_t d = R::template digit_of_item<MODE>(rk, i, keys[i], slot0 + uint32_t(R::kLanes) * i, tvalid, pass, dmask);
-        const uint32_t pos = urow[d] + R::rank_of(rk, i);
+        const uint32_t pos = *R::word(urow, d) + R::rank_of(rk, i);
         stage_k[pos] = keys[i];
         if constexpr (HAS_VAL) stage_v[pos] = vals[i];
     }
@@ -779,8 +823,8 @@ __device__ __forceinline__ void sweep_tile(unsigned char *smem, const SweepTile<
             for (int i = 0; i < ITEMS; ++i) {
                 const uint32_t s = uint32_t(tid) + uint32_t(i) * THREADS;
                 const U k = stage_k[s];
-                const G g = gofs[pass_digit<MODE>(k, pass, dmask)] + G(s);
-                if (uint64_t(g) < n) {
+                const G g = *tile_offset<MODE>(gofs, k, pass, dmask) + G(s);
+                if (inside(g, n)) {
                     if (t.dst_k) t.dst_k[g] = k;
                     if constexpr (HAS_VAL) t.dst_v[g] = stage_v[s];
                 } else {
@@ -790,8 +834,8 @@ __device__ __forceinline__ void sweep_tile(unsigned char *smem, const SweepTile<
         } else {
             for (uint32_t s = tid; s < tvalid; s += THREADS) {
                 const U k = stage_k[s];
-                const G g = gofs[pass_digit<MODE>(k, pass, dmask)] + G(s);
-                if (uint64_t(g) < n) {
+                const G g = *tile_offset<MODE>(gofs, k, pass, dmask) + G(s);
+                if (inside(g, n)) {
                     if (t.dst_k) t.dst_k[g] = k;
                     if constexpr (HAS_VAL) t.dst_v[g] = stage_v[s];
                 } else {
@@ -998,7 +1042,8 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
             tvalidB = uint32_t((n - tbase) < uint64_t(TILE) ? (n - tbase) : uint64_t(TILE));
             load_items<ITEMS, R::kLanes>(keys, src, n, tbase, slot0, tvalidB, TILE, reverse, KeyTraits<U>::fill());
             if constexpr (HAS_VAL) load_items<ITEMS, R::kLanes>(vals, src_v, n, tbase, slot0, tvalidB, TILE, reverse, uint64_t(0));
-            R::template rank<MODE, HOT>(keys, rk, utab, slot0, tvalidB, pass, dmask, hot);
+            if (tvalidB == TILE) R::template rank<MODE, HOT, true, true>(keys, rk, utab, slot0, tvalidB, pass, dmask, hot);
+            else R::template rank<MODE, HOT>(keys, rk, utab, slot0, tvalidB, pass, dmask, hot);
         }
         __syncthreads();                                                        // barrier 1
 
@@ -1074,8 +1119,8 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
                 for (int i = 0; i < ITEMS; ++i) {
                     const uint32_t s = uint32_t(tid) + uint32_t(i) * THREADS;
                     const U k = stage[s];
-                    const G g = gofs[pass_digit<MODE>(k, pass, dmask)] + G(s);
-                    if (uint64_t(g) < n) {
+                    const G g = *tile_offset<MODE>(gofs, k, pass, dmask) + G(s);
+                    if (inside(g, n)) {
                         if (!HAS_VAL || dst) dst[g] = k;
                         if constexpr (HAS_VAL) dst_v[g] = stage_v[s];
                     } else {
@@ -1085,8 +1130,8 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
             } else {
                 for (uint32_t s = tid; s < tvalidA; s += THREADS) {
                     const U k = stage[s];
-                    const G g = gofs[pass_digit<MODE>(k, pass, dmask)] + G(s);
-                    if (uint64_t(g) < n) {
+                    const G g = *tile_offset<MODE>(gofs, k, pass, dmask) + G(s);
+                    if (inside(g, n)) {
                         if (!HAS_VAL || dst) dst[g] = k;
                         if constexpr (HAS_VAL) dst_v[g] = stage_v[s];
                     } else {
@@ -1099,13 +1144,17 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
 
         // ---- (4) stage B sorted by digit (padding slots land past tvalidB); clear the unit words
         if (hasB) {
+            auto place = [&](auto full) {
 #pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                const uint32_t d = R::template digit_of_item<MODE>(rk, i, keys[i], slot0 + uint32_t(R::kLanes) * i, tvalidB, pass, dmask);
-                const uint32_t pos = urow[d] + R::rank_of(rk, i);
-                stage[pos] = keys[i];
-                if constexpr (HAS_VAL) stage_v[pos] = vals[i];
-            }
+                for (int i = 0; i < ITEMS; ++i) {
+                    const uint32_t d = R::template digit_of_item<MODE, decltype(full)::value>(rk, i, keys[i], slot0 + uint32_t(R::kLanes) * i, tvalidB, pass, dmask);
+                    const uint32_t pos = *R::word(urow, d) + R::rank_of(rk, i);
+                    stage[pos] = keys[i];
+                    if constexpr (HAS_VAL) stage_v[pos] = vals[i];
+                }
+            };
+            if (tvalidB == TILE) place(std::true_type{});
+            else place(std::false_type{});
             R::clear_own(utab);
         }
         if (tid == 0) {

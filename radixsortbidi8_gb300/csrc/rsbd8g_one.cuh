@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (int q = 0; q < ITEMS; ++q) {
             if (slot0 + uint32_t(q) * 16u >= tvalid) continue;
             const uint32_t dg = R::template digit_of_item<PM>(rk, q, keys[q], slot0 + uint32_t(q) * 16u, tvalid, p, dm);
-            const uint32_t pos = urow[dg] + R::rank_of(rk, q);
+            const uint32_t pos = *R::word(urow, dg) + R::rank_of(rk, q);
             stage[pos] = keys[q];
             if constexpr (HAS_VAL) stage_v[pos] = vals[q];
         }
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t s = uint32_t(tid) + uint32_t(q) * THREADS;
                 if (s < tvalid) {
                     const U kk = stage[s];
-                    const uint32_t g = uint32_t(gofs[pass_digit<PM>(kk, p, dm)] + int32_t(s));
+                    const uint32_t g = uint32_t(*tile_offset<PM>(gofs, kk, p, dm) + int32_t(s));
                     if (g < n) {
                         if (!HAS_VAL || !last) out_k[g] = kk;
                         if constexpr (HAS_VAL) out_v[g] = stage_v[s];

@@ -588,7 +588,8 @@ __global__ void __launch_bounds__(THREADS, 2)
             const uint64_t tbase = uint64_t(B.tile) * TILE;
             tvalidB = uint32_t((n - tbase) < uint64_t(TILE) ? (n - tbase) : uint64_t(TILE));
             load_items<ITEMS, R::kLanes>(keys, src, n, tbase, slot0, tvalidB, TILE, B.reverse != 0, KeyTraits<U>::fill());
-            R::template rank<MODE>(keys, rk, utab, slot0, tvalidB, pass, B.dmask);
+            if (tvalidB == TILE) R::template rank<MODE, 0, true, true>(keys, rk, utab, slot0, tvalidB, pass, B.dmask);
+            else R::template rank<MODE>(keys, rk, utab, slot0, tvalidB, pass, B.dmask);
         }
         __syncthreads();                                                        // barrier 1
 
@@ -638,19 +639,23 @@ __global__ void __launch_bounds__(THREADS, 2)
             const uint64_t n = A.n;
             for (uint32_t s = tid; s < tvalidA; s += THREADS) {
                 const U k = stage[s];
-                const int32_t g = gofs[pass_digit<MODE>(k, pass, A.dmask)] + int32_t(s);
-                if (uint64_t(g) < n) dst[g] = k;
+                const int32_t g = *tile_offset<MODE>(gofs, k, pass, A.dmask) + int32_t(s);
+                if (inside(g, n)) dst[g] = k;
                 else atomicOr(err_word, kDevFault);     // an offset outside the segment: flagged, not written
             }
         }
         __syncthreads();                                                        // barrier 3
 
         if (hasB) {
+            auto place = [&](auto full) {
 #pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                const uint32_t d = R::template digit_of_item<MODE>(rk, i, keys[i], slot0 + uint32_t(R::kLanes) * i, tvalidB, pass, B.dmask);
-                stage[urow[d] + R::rank_of(rk, i)] = keys[i];
-            }
+                for (int i = 0; i < ITEMS; ++i) {
+                    const uint32_t d = R::template digit_of_item<MODE, decltype(full)::value>(rk, i, keys[i], slot0 + uint32_t(R::kLanes) * i, tvalidB, pass, B.dmask);
+                    stage[*R::word(urow, d) + R::rank_of(rk, i)] = keys[i];
+                }
+            };
+            if (tvalidB == TILE) place(std::true_type{});
+            else place(std::false_type{});
             R::clear_own(utab);
         }
         if (tid == 0) {
