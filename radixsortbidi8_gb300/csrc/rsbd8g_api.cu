@@ -208,6 +208,39 @@ bool device_memory(const void *p) {
     return at.type == cudaMemoryTypeDevice;
 }
 
+// 16-byte keys move as aligned 16-byte words
+static bool misaligned(const Resolved &r, const void *in, const void *out, const void *buf) {
+    if (r.key_bytes != 16 || r.indirect) return false;
+    return ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(buf)) & 15u) != 0;
+}
+
+// the sort as one kernel, if it fits one
+static bool launch_one(const Resolved &r, uint64_t n, unsigned char *sc, size_t bytes, const void *in, void *out, void *buf,
+                       const Layout &L, bool inplace, bool to_buffer, cudaStream_t s, cudaError_t *e) {
+    switch (r.key_bytes) {
+        case 1: return launch_one_k1(r, n, sc, bytes, in, out, buf, L, inplace, to_buffer, s, e);
+        case 2: return launch_one_k2(r, n, sc, bytes, in, out, buf, L, inplace, to_buffer, s, e);
+        case 4: return launch_one_k4(r, n, sc, bytes, in, out, buf, L, inplace, to_buffer, s, e);
+        case 8: return launch_one_k8(r, n, sc, bytes, in, out, buf, L, inplace, to_buffer, s, e);
+        default:
+            return r.x87 ? launch_one_x87(r, n, sc, bytes, in, out, buf, L, inplace, to_buffer, s, e)
+                         : launch_one_k16(r, n, sc, bytes, in, out, buf, L, inplace, to_buffer, s, e);
+    }
+}
+
+// a sort of one tile, without scratch or buffer (*handled false: it needs them)
+static rsbd8g_status enqueue_one_tile(const Resolved &r, uint64_t n, const void *in, void *out, bool inplace, cudaStream_t s,
+                                      bool *handled) {
+    if (n > kOneTileKeys) return RSBD8G_OK;
+    if (misaligned(r, in, out, nullptr)) {
+        *handled = true;
+        return RSBD8G_ERR_BAD_ARG;
+    }
+    cudaError_t e = cudaSuccess;
+    *handled = launch_one(r, n, nullptr, 0, in, out, nullptr, Layout{}, inplace, false, s, &e);
+    return e == cudaSuccess ? RSBD8G_OK : RSBD8G_ERR_CUDA;
+}
+
 rsbd8g_status enqueue_sort(const Resolved &rin, uint64_t n, void *scratch, size_t scratch_bytes, const void *in,
                            void *out, void *buf, bool inplace, bool to_buffer, cudaStream_t s) {
     Resolved r = rin;
@@ -216,22 +249,9 @@ rsbd8g_status enqueue_sort(const Resolved &rin, uint64_t n, void *scratch, size_
     if (!scratch || scratch_bytes < L.total) return RSBD8G_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(scratch) & (kAlign - 1)) != 0) return RSBD8G_ERR_BAD_ARG;
     unsigned char *sc = static_cast<unsigned char *>(scratch);
-    if (r.key_bytes == 16 && !r.indirect) {   // 16-byte keys move as aligned 16-byte words
-        auto mis = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) != 0; };
-        if (mis(in) || (out && mis(out)) || (buf && mis(buf))) return RSBD8G_ERR_BAD_ARG;
-    }
+    if (misaligned(r, in, out, buf)) return RSBD8G_ERR_BAD_ARG;
     cudaError_t e = cudaSuccess;
-    bool one;           // a small sort runs as one kernel
-    switch (r.key_bytes) {
-        case 1: one = launch_one_k1(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
-        case 2: one = launch_one_k2(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
-        case 4: one = launch_one_k4(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
-        case 8: one = launch_one_k8(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e); break;
-        default:
-            one = r.x87 ? launch_one_x87(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e)
-                        : launch_one_k16(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e);
-            break;
-    }
+    const bool one = launch_one(r, n, sc, L.total, in, out, buf, L, inplace, to_buffer, s, &e);   // a small sort
     if (one) return e == cudaSuccess ? RSBD8G_OK : RSBD8G_ERR_CUDA;
     // the scatter passes prefetch tiles into L2 with bulk copies only from device memory
     // (cudaMalloc, memory pools); managed and host memory is read with plain loads alone
@@ -251,6 +271,12 @@ rsbd8g_status enqueue_sort(const Resolved &rin, uint64_t n, void *scratch, size_
     return e == cudaSuccess ? RSBD8G_OK : RSBD8G_ERR_CUDA;
 }
 
+static rsbd8g_status device_status(uint32_t err) {
+    if (err & kDevTimeout) return RSBD8G_ERR_TIMEOUT;
+    if (err & kDevFault) return RSBD8G_ERR_DEVICE_FAULT;
+    return RSBD8G_OK;
+}
+
 rsbd8g_status read_device_status(void *scratch, cudaStream_t s, bool clear) {
     if (!scratch) return RSBD8G_ERR_BAD_ARG;
     uint32_t err = 0;
@@ -262,9 +288,7 @@ rsbd8g_status read_device_status(void *scratch, cudaStream_t s, bool clear) {
         if (cudaMemsetAsync(&ctrl->error, 0, sizeof err, s) != cudaSuccess) return RSBD8G_ERR_CUDA;
         if (cudaStreamSynchronize(s) != cudaSuccess) return RSBD8G_ERR_CUDA;
     }
-    if (err & kDevTimeout) return RSBD8G_ERR_TIMEOUT;
-    if (err & kDevFault) return RSBD8G_ERR_DEVICE_FAULT;
-    return RSBD8G_OK;
+    return device_status(err);
 }
 
 }  // namespace rsbd8g
@@ -460,8 +484,44 @@ static cudaMemPool_t sort_pool() {
     return pools[dev & 63];
 }
 
-// allocating forms: one stream-ordered allocation of buffer + scratch, freed on the stream;
-// the call waits for the sort, as the reference's functions return only when sorted
+// Pinned words that the allocating forms' device status is copied to, so that the copy needs no
+// staging and one synchronisation covers it: one page of them per process, a word per call in flight; a
+// call that finds none free copies to its own stack.
+class StatusWord32 {
+public:
+    StatusWord32() {
+        std::lock_guard<std::mutex> g(mu());
+        if (!page()) {
+            void *p = nullptr;
+            if (cudaHostAlloc(&p, kWords * sizeof(uint32_t), cudaHostAllocPortable) == cudaSuccess) page() = static_cast<uint32_t *>(p);
+            else (void)cudaGetLastError();
+        }
+        if (!page()) return;
+        for (int i = 0; i < kWords && at_ < 0; ++i)
+            if (!((used() >> i) & 1u)) at_ = i;
+        if (at_ >= 0) used() |= uint64_t(1) << at_;
+    }
+    ~StatusWord32() {
+        if (at_ < 0) return;
+        std::lock_guard<std::mutex> g(mu());
+        used() &= ~(uint64_t(1) << at_);
+    }
+    StatusWord32(const StatusWord32 &) = delete;
+    StatusWord32 &operator=(const StatusWord32 &) = delete;
+    uint32_t *word() { return at_ >= 0 ? page() + at_ : &own_; }
+
+private:
+    static constexpr int kWords = 64;
+    static std::mutex &mu() { static std::mutex m; return m; }
+    static uint32_t *&page() { static uint32_t *p = nullptr; return p; }
+    static uint64_t &used() { static uint64_t u = 0; return u; }
+    int at_ = -1;
+    uint32_t own_ = 0;
+};
+
+// allocating forms: one stream-ordered allocation of buffer + scratch, freed on the stream; the call
+// waits for the sort, as the reference's functions return only when sorted.  A sort of one tile takes
+// no memory but its arrays and cannot fail on the device: nothing is allocated or read back.
 static rsbd8g_status sort_alloc(const rsbd8g_desc *desc, size_t count, const void *input, void *output, bool inplace,
                                 rsbd8g_stream stream, const void *keys) {
     Resolved r;
@@ -480,10 +540,16 @@ static rsbd8g_status sort_alloc(const rsbd8g_desc *desc, size_t count, const voi
         return RSBD8G_OK;
     }
     if (!input || (!inplace && (!output || input == output))) return RSBD8G_ERR_BAD_ARG;
+    if (r.flags & RSBD8G_FLAG_DIAG_NOMEM) return RSBD8G_ERR_NO_MEMORY;
+    bool handled = false;
+    st = enqueue_one_tile(r, count, input, output, inplace, s, &handled);
+    if (handled) {
+        if (st == RSBD8G_OK && cudaStreamSynchronize(s) != cudaSuccess) st = RSBD8G_ERR_CUDA;
+        return st;
+    }
     const Layout L = layout_for(r, count);
     const size_t buf_bytes = (size_t(count) * r.elem_bytes + 255) & ~size_t(255);
     void *mem = nullptr;
-    if (r.flags & RSBD8G_FLAG_DIAG_NOMEM) return RSBD8G_ERR_NO_MEMORY;
     cudaMemPool_t pool = sort_pool();
     const cudaError_t ae = pool ? cudaMallocFromPoolAsync(&mem, L.total + buf_bytes, pool, s)
                                 : cudaMallocAsync(&mem, L.total + buf_bytes, s);
@@ -494,11 +560,14 @@ static rsbd8g_status sort_alloc(const rsbd8g_desc *desc, size_t count, const voi
     unsigned char *scratch = static_cast<unsigned char *>(mem);
     void *buffer = scratch + L.total;
     st = enqueue_sort(r, count, scratch, L.total, input, inplace ? nullptr : output, buffer, inplace, false, s);
-    rsbd8g_status dev = RSBD8G_OK;
-    if (st == RSBD8G_OK) dev = read_device_status(scratch, s, false);
+    StatusWord32 status;
+    *status.word() = 0;
+    if (st == RSBD8G_OK && cudaMemcpyAsync(status.word(), &reinterpret_cast<Control *>(scratch)->error, sizeof(uint32_t),
+                                           cudaMemcpyDeviceToHost, s) != cudaSuccess)
+        st = RSBD8G_ERR_CUDA;
     cudaFreeAsync(mem, s);
     if (cudaStreamSynchronize(s) != cudaSuccess && st == RSBD8G_OK) st = RSBD8G_ERR_CUDA;
-    return st != RSBD8G_OK ? st : dev;
+    return st != RSBD8G_OK ? st : device_status(*status.word());
 }
 
 RSBD8G_API rsbd8g_status rsbd8g_radixsortcopy(const rsbd8g_desc *desc, size_t count, const void *input, void *output,

@@ -94,6 +94,9 @@ RSBD8G_DECLARE_ONE(launch_one_k8)
 RSBD8G_DECLARE_ONE(launch_one_k16)
 RSBD8G_DECLARE_ONE(launch_one_x87)
 
+// the largest sort that one tile holds (rsbd8g_onelaunch.cuh); such a sort uses neither scratch nor buffer
+constexpr uint64_t kOneTileKeys = 4096;
+
 // tile geometry of the onesweep passes, per key size (keys per tile = threads * items)
 struct SweepGeometry {
     int threads, items;

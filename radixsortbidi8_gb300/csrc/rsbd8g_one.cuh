@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t tvalid = n - base < uint32_t(TILE) ? n - base : uint32_t(TILE);
     const uint32_t dm = HAS_VAL ? 0u : a.dmask;
     const uint32_t slot0 = R::slot0();
-    if (G == 1 && tid == 0) ctrl->error = 0;
+    if (G == 1 && tid == 0 && ctrl) ctrl->error = 0;
     uint32_t bar = 0;
 
     // ---- load the tile, count every digit
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (G > 1 && last && dst == cur && !one_barrier(ctrl, bar += G, a.spin_limit_ns, misc + 32)) return;
         if (G > 1 || last) {
             const uint32_t dk = curk == kArrKeysA ? kArrKeysB : kArrKeysA;
-            U *out_k = static_cast<U *>(sort_array(arrs, HAS_VAL ? dk : dst, kArrBuf, &bad_arr));
+            U *out_k = HAS_VAL && last ? nullptr : static_cast<U *>(sort_array(arrs, HAS_VAL ? dk : dst, kArrBuf, &bad_arr));
             uint64_t *out_v = static_cast<uint64_t *>(sort_array(arrs, dst, kArrBuf, &bad_arr));
 #pragma unroll
             for (int q = 0; q < ITEMS; ++q) {
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (g < n) {
                         if (!HAS_VAL || !last) out_k[g] = kk;
                         if constexpr (HAS_VAL) out_v[g] = stage_v[s];
-                    } else {
+                    } else if (ctrl) {
                         atomicOr(&ctrl->error, kDevFault);
                     }
                 }

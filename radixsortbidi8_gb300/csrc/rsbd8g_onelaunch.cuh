@@ -28,6 +28,8 @@ constexpr OneShape one_shape(int key_bytes, bool indirect, int i) {
                     : OneShape{1024, !indirect && key_bytes <= 4 ? 16 : 0};
 }
 
+static_assert(kOneTileKeys == 1024 * 4, "the larger of the two sizes that sort in one tile");
+
 // set the kernel up on device `dev` (which also loads it); returns the CTAs that fit the device at once
 template <typename U, int MODE, bool HAS_VAL, int SHAPE>
 uint64_t one_setup(int dev) {
@@ -69,7 +71,7 @@ bool launch_one_shape(const OneCall &c, uint64_t most, cudaError_t *e) {
         const size_t used = status + size_t(tiles + tiles / kOneGroup) * kBuckets * 4;
         int dev = 0;
         cudaGetDevice(&dev);
-        if (used > c.scratch_bytes || tiles > most || tiles > one_setup<U, MODE, HAS_VAL, SHAPE>(dev)) return false;
+        if ((tiles > 1 && used > c.scratch_bytes) || tiles > most || tiles > one_setup<U, MODE, HAS_VAL, SHAPE>(dev)) return false;
         if (tiles > 1) {
             LaunchTimer t(c.s, RSBD8G_KERNEL_MEMSET, uint32_t(sizeof(U)), 0, c.n);
             if ((*e = cudaMemsetAsync(c.scratch, 0, used, c.s)) != cudaSuccess) return true;
@@ -86,8 +88,8 @@ bool launch_one_shape(const OneCall &c, uint64_t most, cudaError_t *e) {
         cfg.attrs = &at;
         cfg.numAttrs = tiles > 1 ? 1 : 0;
         *e = cudaLaunchKernelEx(&cfg, k_sort_one<U, MODE, HAS_VAL, sh.threads, sh.items>, reinterpret_cast<Control *>(c.scratch), c.arrs,
-                                reinterpret_cast<uint32_t *>(c.scratch + hist),
-                                reinterpret_cast<uint32_t *>(c.scratch + status), c.args);
+                                tiles > 1 ? reinterpret_cast<uint32_t *>(c.scratch + hist) : nullptr,
+                                tiles > 1 ? reinterpret_cast<uint32_t *>(c.scratch + status) : nullptr, c.args);
         return true;
     }
 }
@@ -108,7 +110,8 @@ bool launch_one_mode(const OneCall &c, cudaError_t *e) {
            launch_one_shape<U, MODE, HAS_VAL, 3>(c, ~uint64_t(0), e);
 }
 
-// Run the sort as one kernel if it fits; false (nothing launched) if it does not.
+// Run the sort as one kernel if it fits; false (nothing launched) if it does not.  A sort of one tile may
+// come without scratch and buffer.
 template <typename U>
 bool launch_one_t(const Resolved &r, uint64_t n, unsigned char *scratch, size_t scratch_bytes, const void *in, void *out,
                   void *buf, const Layout &L, bool inplace, bool to_buffer, cudaStream_t s, cudaError_t *e) {
@@ -121,8 +124,10 @@ bool launch_one_t(const Resolved &r, uint64_t n, unsigned char *scratch, size_t 
     c.arrs.p[kArrIn] = in;
     c.arrs.p[kArrOut] = out;
     c.arrs.p[kArrBuf] = buf;
-    c.arrs.p[kArrKeysA] = r.indirect ? scratch + L.keys_a : nullptr;
-    c.arrs.p[kArrKeysB] = r.indirect ? scratch + L.keys_b : nullptr;
+    if (scratch && r.indirect) {
+        c.arrs.p[kArrKeysA] = scratch + L.keys_a;
+        c.arrs.p[kArrKeysB] = scratch + L.keys_b;
+    }
     c.args.n = n;
     c.args.spin_limit_ns = 1000000000ull;
     c.args.inplace = inplace;
