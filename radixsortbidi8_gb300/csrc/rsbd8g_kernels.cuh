@@ -249,10 +249,20 @@ __global__ void __launch_bounds__(THREADS) k_histogram(const U *__restrict__ key
     plan_if_last<THREADS>(ctrl, ghist, bstart, n, pa);
 }
 
+// key i of an indirect sort (as k_gather_histogram loads it; that kernel keeps its own copy in line, where
+// the loads of four keys are in flight together)
+template <typename U>
+__device__ __noinline__ U gathered_key(const uint64_t *ptrs, uint64_t i, int64_t off1, int64_t off2, int level, const U *keys_in) {
+    if (level == 3) return keys_in[i];
+    const unsigned char *obj = reinterpret_cast<const unsigned char *>(ptrs[i]) + off1;
+    if (level == 2) obj = load_ptr(obj) + off2;
+    return load_member<U>(obj);
+}
+
 // indirect form: gather the key through each object pointer (level 1: at off1; level 2: behind the
 // pointer held at off1, at off2; level 3: keys_in[i], supplied by the caller), write the filtered key
 template <typename U, int MODE, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_gather_histogram(const uint64_t *__restrict__ ptrs, uint64_t n,
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS) k_gather_histogram(const uint64_t *__restrict__ ptrs, uint64_t n,
                                                               uint32_t dmask, int64_t off1, int64_t off2, int level,
                                                               const U *__restrict__ keys_in,
                                                               U *__restrict__ keys_out,
@@ -261,15 +271,11 @@ __global__ void __launch_bounds__(THREADS) k_gather_histogram(const uint64_t *__
                                                               unsigned long long *__restrict__ bstart, PlanArgs pa) {
     constexpr int P = KeyTraits<U>::kDigits;
     __shared__ __align__(16) uint32_t shall[gather_hist_copies<P>() * P * kBuckets];
-    auto key_at = [&](uint64_t i) {
-        if (level == 3) return keys_in[i];
-        const unsigned char *obj = reinterpret_cast<const unsigned char *>(ptrs[i]) + off1;
-        if (level == 2) obj = load_ptr(obj) + off2;
-        return load_member<U>(obj);
-    };
     if constexpr (P >= 8) {
         if (pa.prefix_ok)
-            prefix_sample_cta<U, THREADS>(reinterpret_cast<U *>(shall), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(key_at(i)); });
+            prefix_sample_cta<U, THREADS>(reinterpret_cast<U *>(shall), n, ctrl, [&](uint64_t i) {
+                return filter_key<MODE>(gathered_key<U>(ptrs, i, off1, off2, level, keys_in));
+            });
     }
     zero_hist<THREADS, P>(shall);
     uint32_t *sh = shall + ((threadIdx.x >> 5) % gather_hist_copies<P>()) * P * kBuckets;
@@ -283,7 +289,15 @@ __global__ void __launch_bounds__(THREADS) k_gather_histogram(const uint64_t *__
         for (int u = 0; u < UNR; ++u) {
             const uint64_t i = b + u * 32 + lane;
             raw[u] = U{};
-            if (i < n) raw[u] = key_at(i);
+            if (i < n) {
+                if (level == 3) {
+                    raw[u] = keys_in[i];
+                } else {
+                    const unsigned char *obj = reinterpret_cast<const unsigned char *>(ptrs[i]) + off1;
+                    if (level == 2) obj = load_ptr(obj) + off2;
+                    raw[u] = load_member<U>(obj);
+                }
+            }
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
