@@ -26,6 +26,13 @@ struct Resolved {
     const void *keys;     // RSBD8G_KEYED: the caller's key array
 };
 
+// Resolved::flags of a batch whose kernels share the GPU with other streams' (the server sets it): it is not
+// sorted by a prefix, as the launches that leaves idle would each wait for their CTAs' turn behind
+// another stream's passes (29 mixed requests of up to 2^22 keys: 1.22-1.29 ms with them, 1.11 without; one
+// large request alone still gains more than it waits: 48 requests of up to 2^24 keys 2.85 ms, 3.07 without).
+// The same bit is named in rsbd8g_serve.cpp.
+constexpr uint32_t kFlagSharedGpu = 1u << 30;
+
 // byte offsets of the parts of a scratch area
 struct Layout {
     size_t ctrl, ghist, bstart, status, status_pass_bytes, zero_bytes, keys_a, keys_b, total;

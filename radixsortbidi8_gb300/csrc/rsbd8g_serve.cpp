@@ -36,6 +36,7 @@ int filter_class(const rsbd8g_desc *d);       // rsbd8g_api.cu
 namespace {
 
 constexpr size_t kAlignArena = 256;
+constexpr uint32_t kFlagSharedGpu = 1u << 30;     // rsbd8g_internal.h
 size_t aup(size_t x) { return (x + kAlignArena - 1) & ~(kAlignArena - 1); }
 
 // first-fit allocator over [0, size) of the arena; host bookkeeping only
@@ -335,6 +336,7 @@ struct Server {
         bool device = true;
         for (size_t i = 0; i < n; ++i) device = device && b->reqs[i]->device;
         if (device) key.flags |= RSBD8G_FLAG_DEVICE_ARRAYS;
+        key.flags |= kFlagSharedGpu;       // (batches overlap on the device)
         for (size_t i = 0; i < n; ++i) {
             ho[i + 1] = ho[i] + b->reqs[i]->count;
             hi[i] = reinterpret_cast<uint64_t>(b->reqs[i]->in);
