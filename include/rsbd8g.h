@@ -318,8 +318,10 @@ RSBD8G_API const char *rsbd8g_status_string(rsbd8g_status status);
 
 /* ---- launch profiling (measurement support; no counterpart in the reference) ---------- */
 
-/* The plain sorts compute their plan in the histogram launch, so PLAN records only the segmented
- * sort's plan launch. The copy forms fold the copy step into the last digit pass, so COPY records the
+/* A plain sort that fits the device's tiles is one kernel (ONE). The others compute their plan in the
+ * histogram launch, so PLAN records only the segmented sort's plan launch. SETTLE records the step that
+ * completes sorts of 8- and 16-byte keys by a prefix of their digits; passes that the plan leaves out
+ * are recorded too (they return at once). The copy forms fold the copy step into the last digit pass, so COPY records the
  * in-place forms' copy launch and the segmented sort's. */
 enum {
     RSBD8G_KERNEL_MEMSET = 0, RSBD8G_KERNEL_HISTOGRAM = 1, RSBD8G_KERNEL_PLAN = 2,
@@ -330,7 +332,7 @@ enum {
 typedef struct rsbd8g_launch_record {
     uint32_t kernel;      /* RSBD8G_KERNEL_* */
     uint32_t key_bytes;
-    uint32_t pass;        /* digit index of an onesweep launch */
+    uint32_t pass;        /* position of an onesweep launch in the sort: the digit, or the n-th pass slot of wide keys */
     uint32_t reserved;
     uint64_t count;       /* elements of the sort the launch belongs to */
     double ms;            /* device time between CUDA events recorded around the launch on its stream */

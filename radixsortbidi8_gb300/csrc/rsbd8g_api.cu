@@ -2,9 +2,10 @@
 //
 // Mode resolution restates helper::isabsvalue / issignmode / isfltpmode / isdescsort /
 // isrevorderwithindirection / isrevorderwithoutindirection (Radixsortbidi8.hpp:59778-59904);
-// the call sequence per sort is
+// the call sequence per sort is one kernel for a small sort (rsbd8g_onelaunch.cuh), else
 //   memset(control, histograms, look-back state) -> histogram (or gather+histogram)
-//   -> plan (scan + pass-skip + ping-pong) -> one onesweep pass per digit -> copy step,
+//   -> plan (scan + pass-skip + ping-pong) -> one onesweep pass per digit (wide keys: over a prefix
+//   of the digits, then the settle step) -> copy step,
 // all on the caller's stream, with no host synchronisation in between (a skipped pass
 // returns at once on the device), so the sequence can be captured in a CUDA graph.
 #include <cuda_runtime.h>

@@ -121,9 +121,9 @@ constexpr SweepGeometry sweep_geometry(int key_bytes, bool indirect) {
 constexpr uint64_t kLargeTileMinKeys = uint64_t(1) << 25;
 constexpr uint64_t kSmallTileMaxKeys = uint64_t(1) << 23;
 // Sorts of 8- and 16-byte keys from this many keys on may run as prefix sorts (rsbd8g_prefix.cuh): below,
-// the launches of a plain sort that a prefix sort leaves idle cost more than the passes it saves
-// (int64 2^20: 137 us plain, 130-142 us as a prefix sort; 2^21: 182 and 152-170 us; 128-bit 2^20: 320
-// and 203 us).
+// the launches that a prefix sort leaves idle cost what the passes it saves do (8-byte keys 2^20: 137 us
+// plain, 130-142 us by a prefix, and 91 us as one kernel; 2^21: 182 and 111-132 us; 128-bit 2^20: 320 and
+// 137 us).
 constexpr uint64_t prefix_min_keys(int key_bytes) { return uint64_t(1) << (key_bytes == 16 ? 20 : 21); }
 constexpr SweepGeometry sweep_geometry_large(int key_bytes) {
     return key_bytes <= 4 ? SweepGeometry{512, 32} : sweep_geometry(key_bytes, false);

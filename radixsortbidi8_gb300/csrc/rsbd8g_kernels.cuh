@@ -17,6 +17,8 @@
 //   k_onesweep_pipe                    the same pass with the look-back of one tile overlapping the
 //                                      load and ranking of the next, and the next tile prefetched
 //                                      into L2 (the pass of every sort of two tiles per CTA or more)
+//   (8- and 16-byte keys: the passes may stop at a prefix of the digits, which k_settle completes,
+//    rsbd8g_prefix.cuh; sorts that fit the SMs' tiles run as one kernel, rsbd8g_one.cuh)
 //   k_copy                             the plain / reversed copy of the in-place forms when parity
 //                                      or all-skipped passes need one (the copy forms need one only
 //                                      when every pass was skipped, and the last pass's launch does it)

@@ -6,7 +6,10 @@
 //   the last of which also runs the copy step of the copy forms -> copy step (in-place forms only)
 // all on the caller's stream, with no host synchronisation in between (a skipped pass returns at
 // once on the device), so the sequence can be captured in a CUDA graph: 2 + digits launches for
-// the copy forms, 3 + digits for the in-place forms.
+// the copy forms, 3 + digits for the in-place forms.  Large sorts of 8- and 16-byte keys take
+// kPrefixSlots pass launches and the settle step ahead of one launch per digit (rsbd8g_prefix.cuh);
+// those that the plan leaves idle return at once.  Each launch after the histogram may start while the
+// one before it drains (launch_after).  Small sorts run as one kernel instead (rsbd8g_onelaunch.cuh).
 #pragma once
 #include <algorithm>
 #include <mutex>

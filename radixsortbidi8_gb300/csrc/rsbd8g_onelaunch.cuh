@@ -90,6 +90,12 @@ bool launch_one_shape(const OneCall &c, uint64_t most, cudaError_t *e) {
         *e = cudaLaunchKernelEx(&cfg, k_sort_one<U, MODE, HAS_VAL, sh.threads, sh.items>, reinterpret_cast<Control *>(c.scratch), c.arrs,
                                 tiles > 1 ? reinterpret_cast<uint32_t *>(c.scratch + hist) : nullptr,
                                 tiles > 1 ? reinterpret_cast<uint32_t *>(c.scratch + status) : nullptr, c.args);
+        if (*e == cudaErrorCooperativeLaunchTooLarge || *e == cudaErrorNotSupported) {
+            // a context that may not use every SM: the launches per digit need no CTAs side by side
+            (void)cudaGetLastError();
+            *e = cudaSuccess;
+            return false;
+        }
         return true;
     }
 }

@@ -8,10 +8,13 @@
 //                    LSD radix sort over 8-bit digits with the same warp multisplit and the
 //                    reference's pass-skip test per segment
 //   k_seg_hist       per large segment, all digit histograms in one read (tiles in order)
-//   k_seg_plan       per large segment: exclusive scans, pass-skip mask
+//   k_seg_plan       per large segment: exclusive scans, pass-skip mask (k_seg_plan_wide: 8- and 16-byte
+//                    keys, which also samples the segment and may choose a prefix of its digits)
 //   k_seg_sweep      one onesweep pass over the tiles of every large segment: look-back chains
 //                    stay inside a segment; each segment ping-pongs by its own surviving passes
 //                    (k_seg_sweep_pipe: the same pass with the look-back one tile behind)
+//   k_seg_settle     the segments sorted by a prefix completed in place; those it cannot settle take
+//                    the sweeps of phase 1 (rsbd8g_prefix.cuh)
 //   k_seg_copy       large segments whose every digit was skipped (plain or reversed copy)
 #pragma once
 #include "rsbd8g_kernels.cuh"

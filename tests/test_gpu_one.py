@@ -85,7 +85,7 @@ def test_pointers(dtype, direction, n):
     assert np.array_equal(ptr.cpu().numpy(), want)
 
 
-@pytest.mark.parametrize("n", [2048, 100003])
+@pytest.mark.parametrize("n", [2048, 100003, (1 << 22) + 3])      # one tile, several, a launch per digit
 def test_captured_in_a_graph(n):
     import torch
     import radixsortbidi8_gb300 as rs
