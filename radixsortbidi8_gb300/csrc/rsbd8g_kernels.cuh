@@ -432,9 +432,9 @@ constexpr int rank_lanes() { return ITEMS >= 16 ? 16 : 32; }
 
 // DENSE packs the ranks of large tiles as tightly as the unit size allows and advances a half-warp
 // unit's count with a plain store (the same word the add would leave: no other lane writes it before
-// the next item).  It pays only where registers are scarcest: the segmented pass over 8-byte keys
-// (batch of 20,000 arrays: -3.2 %, spills 36 -> 20 bytes); on the plain sorts it measured within
-// +-0.6 % of the default, a net loss on the mixed workload.
+// the next item).  It pays for 8-byte keys: the segmented pass (batch of 20,000 arrays: -3.2 %, spills
+// 36 -> 20 bytes) and, with scaled digits, the plain one (eight passes over 2^26 int64 keys 2.582 -> 2.560
+// ms); keys of up to 4 bytes measured within +-0.6 % of the default, a net loss on the mixed workload.
 template <int THREADS, int ITEMS, int LANES = rank_lanes<ITEMS>(), bool DENSE = false>
 struct TileRank {
     static_assert(LANES == 16 || LANES == 32, "half-warp or warp units");
@@ -983,7 +983,7 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
                                                    uint32_t dmask) {
     using L = PipeSmem<U, THREADS, ITEMS, HAS_VAL>;
     constexpr int TILE = L::kTile;
-    using R = TileRank<THREADS, ITEMS>;
+    using R = TileRank<THREADS, ITEMS, rank_lanes<ITEMS>(), sizeof(U) == 8>;   // dense ranks: 8-byte keys
     const uint32_t hot = plan.hot;
     U *stage = reinterpret_cast<U *>(smem);
     uint64_t *stage_v = reinterpret_cast<uint64_t *>(smem + L::kOffV);
@@ -1131,7 +1131,8 @@ __device__ __forceinline__ void onesweep_pipe_body(unsigned char *smem, Control 
         }
         if (hasA && misc[1] == 0u && tileA != stall_tile) {
             if (tvalidA == TILE) {
-#pragma unroll 4
+                constexpr int kUnroll = sizeof(U) == 8 ? 8 : 4;      // (8-byte keys: 0.4 % faster than 4)
+#pragma unroll kUnroll
                 for (int i = 0; i < ITEMS; ++i) {
                     const uint32_t s = uint32_t(tid) + uint32_t(i) * THREADS;
                     const U k = stage[s];
