@@ -107,6 +107,18 @@ struct Control {
 };
 static_assert(sizeof(Control) <= 1024, "control block must fit its slot");
 
+// The plan's numbers that place an access are checked where they are read, as the array indices are
+// (sort_array): a pass's digit and look-back array, the prefix of a settle step, and the digits of the
+// passes it plans.  One that is out of range sets the fault flag and nothing is accessed.
+template <int DIGITS>
+__host__ __device__ __forceinline__ bool plan_in_range(const PassPlan &p) {
+    return p.digit < DIGITS && p.status < DIGITS;
+}
+template <int DIGITS>
+__host__ __device__ __forceinline__ bool prefix_in_range(uint32_t passes, uint32_t low, uint32_t survive) {
+    return passes <= uint32_t(kPrefixSlots) && low < uint32_t(DIGITS) && (survive >> DIGITS) == 0;
+}
+
 // ---- key filter -----------------------------------------------------------------------
 
 // K(b): transform raw key bits into an unsigned key whose ascending order is the reference's

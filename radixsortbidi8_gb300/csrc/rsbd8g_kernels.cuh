@@ -936,6 +936,10 @@ __global__ void __launch_bounds__(THREADS, onesweep_min_blocks<U, HAS_VAL, THREA
         if (fold_copy) copy_step(ctrl, arrs, n, HAS_VAL ? 8u : uint32_t(sizeof(U)));
         return;
     }
+    if (KeyTraits<U>::kDigits >= 8 && !plan_in_range<KeyTraits<U>::kDigits>(plan)) {    // a damaged control block
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&ctrl->error, kDevFault);
+        return;
+    }
     // keys of up to 4 bytes sort by digit `slot` in launch `slot`; the plan of wider keys names the digit
     const int pass = KeyTraits<U>::kDigits >= 8 ? int(plan.digit) : slot;
     S *status = status_all + status_stride * (KeyTraits<U>::kDigits >= 8 ? uint32_t(plan.status) : 0u);
@@ -1201,6 +1205,10 @@ __global__ void __launch_bounds__(THREADS, 2)
     if (!plan.active) {
         // the last pass of a copy form: when every pass was skipped, the copy the plan asks for
         if (fold_copy) copy_step(ctrl, arrs, n, HAS_VAL ? 8u : uint32_t(sizeof(U)));
+        return;
+    }
+    if (KeyTraits<U>::kDigits >= 8 && !plan_in_range<KeyTraits<U>::kDigits>(plan)) {    // a damaged control block
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&ctrl->error, kDevFault);
         return;
     }
     // keys of up to 4 bytes sort by digit `slot` in launch `slot`; the plan of wider keys names the digit

@@ -145,10 +145,12 @@ __device__ __forceinline__ uint32_t prefix_choose(const uint32_t *sample_pairs, 
 // slots from slot0.  A copy form must end in its output; `even` makes the number of passes even (by
 // sorting by the lowest digit twice) for a chain that starts there.  keep_keys: the last pass of an
 // indirect sort writes its keys too; hot: the crowded digit of each position.  One thread calls it.
-__device__ __forceinline__ uint32_t plan_chain(Control *__restrict__ ctrl, const PlanArgs &a, const uint32_t *hot, uint32_t mask, bool even,
+__host__ __device__ __forceinline__ uint32_t plan_chain(Control *__restrict__ ctrl, const PlanArgs &a, const uint32_t *hot, uint32_t mask, bool even,
                                                int slot0, uint32_t cur, uint32_t &curk, bool rev, bool keep_keys) {
-    const int again = even && (__popc(mask) & 1) ? 1 : 0;
-    const int k = __popc(mask) + again;
+    int digits = 0;
+    for (uint32_t m = mask; m; m &= m - 1) ++digits;
+    const int again = even ? digits & 1 : 0;
+    const int k = digits + again;
     int p = -1;
     for (int i = 1; i <= k; ++i) {
         if (!(again && i == 2)) {
@@ -483,14 +485,14 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
     constexpr int THREADS = S::kThreads, C = S::kChunk;
     next_may_start();
     after_previous();
-    const uint32_t k = ctrl->prefix_passes;
+    const uint32_t k = ctrl->prefix_passes, low = ctrl->prefix_low, survive = ctrl->survive;
     if (k == 0 || ctrl->abort) return;
     __shared__ __align__(16) U keys_s[S::kWarps][S::kView];
     __shared__ uint32_t words_s[S::kWarps][2][S::kWords];
     __shared__ uint32_t last;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const PassPlan &end = ctrl->plan[k - 1];
-    bool bad = false;
+    bool bad = !prefix_in_range<KeyTraits<U>::kDigits>(k, low, survive);
+    const PassPlan end = ctrl->plan[bad ? 0u : k - 1];
     U *keys = static_cast<U *>(sort_array(arrs, end.dst_keys, HAS_VAL ? kArrKeysA : kArrBuf, &bad));
     uint64_t *vals = static_cast<uint64_t *>(sort_array(arrs, end.dst_vals, kArrBuf, &bad));
     if (bad || !keys || (HAS_VAL && !vals)) {       // a damaged control block
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
     // the prefix passes' look-back words, cleared for the plain passes that a failure calls for
     for (uint64_t i = uint64_t(blockIdx.x) * THREADS + tid; i < uint64_t(k) * status_bytes / 16; i += uint64_t(gridDim.x) * THREADS)
         reinterpret_cast<uint4 *>(status)[i] = make_uint4(0, 0, 0, 0);
-    const U mask = prefix_mask<U>(ctrl->prefix_low);
+    const U mask = prefix_mask<U>(low);
     const uint64_t chunks = (n + C - 1) / C, stride = uint64_t(gridDim.x) * S::kWarps;
     uint32_t seen = 0;
     for (uint64_t c = uint64_t(blockIdx.x) * S::kWarps + warp; c < chunks; c += stride) {
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
     // a group was too long to settle: the plain passes, over every digit, from where the data stand
     const uint32_t cur = HAS_VAL ? end.dst_vals : end.dst_keys;
     uint32_t curk = end.dst_keys;
-    const uint32_t done = plan_chain(ctrl, pa, ctrl->hot, ctrl->survive, !pa.inplace, kPrefixSlots, cur, curk, false, false);
+    const uint32_t done = plan_chain(ctrl, pa, ctrl->hot, survive, !pa.inplace, kPrefixSlots, cur, curk, false, false);
     plan_copy(ctrl, pa, done, false);
 }
 

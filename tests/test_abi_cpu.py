@@ -132,6 +132,22 @@ def test_sort_array_lookup_of_the_control_block_indices(tmp_path):
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
 
 
+def test_plan_numbers_from_scratch_are_in_range(tmp_path):
+    """The digit, look-back array and prefix that the kernels read from the control block name what the sort
+    has, or are refused (rsbd8g::plan_in_range, prefix_in_range), checked on the host."""
+    import shutil
+    import subprocess
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    exe = str(tmp_path / "plan_range_test")
+    r = subprocess.run([nvcc, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "radixsortbidi8_gb300", "csrc"),
+                        os.path.join(ROOT, "tests", "cpp", "plan_range_test.cu"), "-o", exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
 def test_prepare_and_tuning_refusals_without_a_device():
     """rsbd8g_prepare refuses a bad descriptor before touching the device; the segmented scratch
     sizing refuses a small shape or large-segment tile that was not compiled."""
