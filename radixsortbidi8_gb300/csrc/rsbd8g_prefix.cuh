@@ -12,10 +12,9 @@
 //                     all of them, are needed: then the plain LSD passes run
 //   * k_settle        puts every group of equal prefixes into the order of the whole keys, ties in
 //                     the order they came (the passes were stable), so the result is the LSD sort's
-//                     bit for bit.  A group that is already in order, whatever its length, costs
-//                     nothing; one that is out of order and longer than a warp's view sets
-//                     settle_fail, and the plain passes over every digit then sort the array as it
-//                     stands: still a stable arrangement of the input, with the same histograms.
+//                     bit for bit.  One that is out of order and longer than the samples let pass
+//                     (settle_limit) sets settle_fail, and the plain passes over every digit then sort the
+//                     array as it stands: still a stable arrangement of the input, with the same histograms.
 // Everything is decided on the device, so a sort still never synchronises with the host.
 #pragma once
 #include "rsbd8g_device.cuh"
@@ -218,11 +217,13 @@ __device__ __forceinline__ void plan_copy(Control *__restrict__ ctrl, const Plan
 // keys keep their order): a round per key that another has to pass, a few for groups of a few keys.
 //   A group that is still open at the end of the halo, or takes more than kRounds rounds, is settled by
 // the warp in shared memory, with kView keys in view, every key moving to the place found by comparing
-// it with its group.  A group from an earlier chunk is left alone, so an inversion in one raises
-// settle_fail unless the chunk before this one holds its start and this one's first kReach keys hold
-// the inversion; and so does an inversion in a group that runs past kView.  So no inversion is passed over.
-// Neighbouring chunks read keys that a chunk moves only for their prefixes, which a move within a
-// group leaves as they are.
+// it with its group (settle_wide).  One that runs past the view is settled by the first warp that meets an inversion
+// in it, whichever chunk that is in, after its chunks: by digit passes of its own over the digits below the prefix,
+// through the array that the scatter passes left free (settle_long).
+//   A group from an earlier chunk is otherwise left alone, as that chunk's warp settles it.  No inversion is passed
+// over: each lies in some warp's chunk, and its group either ends within the view of the chunk it starts in
+// or is taken by settle_long, which raises settle_fail where the group is too long.  Neighbouring chunks read keys
+// that a chunk moves only for their prefixes, which a move within a group leaves as they are.
 template <typename U>
 struct SettleShape {
     static constexpr int kThreads = sizeof(U) == 8 ? 256 : 128;     // (static shared memory stays below 48 KB)
@@ -230,11 +231,46 @@ struct SettleShape {
     static constexpr int kItems = 8;
     static constexpr int kChunk = 31 * kItems;
     static constexpr int kCtaKeys = kWarps * kChunk;
-    static constexpr int kReach = 224;
-    static constexpr int kView = kChunk + kReach;
+    static constexpr int kView = kChunk + 224;
     static constexpr int kWords = (kView + 31) / 32;
     static constexpr int kRounds = 12;
 };
+
+// The longest group of n keys that a warp settles: 2 sqrt(n) keys, rounded up.  A crowd of g keys among
+// spread ones shows as (g / n)^2 of the samples' pairs, which prefix_choose takes for too many from g =
+// sqrt(2 n) on, give or take the few pairs that make the difference; so a longer group that no sample saw is
+// rare, and one as long as this costs far less than the plain passes would (2^28 int64 keys, 10,000 of them one
+// group: 6.2 ms, 14.9 with the plain passes and 5.9 without such a group; 2^21 keys, 500: 152, 274 and 131 us).
+__host__ __device__ __forceinline__ uint64_t settle_limit(uint64_t n) {
+    int bits = 0;
+    while (bits < 40 && (uint64_t(1) << bits) < n) ++bits;
+    const uint64_t m = uint64_t(1) << ((bits + 1) / 2 + 1);
+    return m < 1024 ? 1024 : m;
+}
+
+// Inversions in long groups that a warp keeps (more fail the step: crowds are for the samples to see); with 24, the
+// five CTAs of an SM passed 164 KB of shared memory and L1 halved: 2^28 keys 594 -> 624 us.
+constexpr uint32_t kSettleLater = 12;
+// a warp's shared memory in the settle step
+template <typename U>
+struct alignas(16) SettleWarp {
+    U key[SettleShape<U>::kView];
+    uint32_t head[SettleShape<U>::kWords], inv[SettleShape<U>::kWords];
+    // inversions found in long groups (tag + place), for settle_long after the warp's chunks
+    uint32_t found;
+    uint64_t later[kSettleLater], tag;
+};
+// what settle_long needs beside the keys: the arrays that are free, the long groups that were taken up (a hash table
+// of start + tag + 1, 0 for none), settle_limit, and the surviving digits below the prefix
+template <typename U>
+struct SettleLong {
+    U *free_keys;
+    uint64_t *free_vals;
+    unsigned long long *taken;
+    uint64_t tag, limit;
+    uint32_t room, digits;
+};
+constexpr uint32_t kTakenRoom = 4096;      // entries of the table, at most
 
 // the last set bit of w[] at or below position i, -1 if there is none
 __device__ __forceinline__ int bit_at_or_below(const uint32_t *w, int i) {
@@ -275,11 +311,187 @@ __device__ __forceinline__ U settle_order(U b, bool desc) {
     return desc ? key_not(q) : q;
 }
 
+// take up the long group `id`: 1, or 0 if another warp has, -1 if the table is full
+template <typename U>
+__device__ __forceinline__ int settle_take(const SettleLong<U> &w, unsigned long long id) {
+    if (w.room == 0) return -1;
+    uint32_t h = uint32_t((id * 0x9E3779B97F4A7C15ull) >> 32) % w.room;
+    for (int i = 0; i < 64; ++i) {
+        const unsigned long long old = atomicCAS(w.taken + h, 0ull, id);
+        if (old == 0ull) return 1;
+        if (old == id) return 0;
+        h = h + 1 == w.room ? 0 : h + 1;
+    }
+    return -1;
+}
+
+// keep an inversion in a long group for settle_long (of the lanes that call it at once, the first one's)
+template <typename U>
+__device__ __noinline__ void settle_later(SettleWarp<U> *warp, uint64_t at, uint32_t *fail, uint32_t fail_bit) {
+    if ((threadIdx.x & 31u) != uint32_t(__ffs(__activemask()) - 1)) return;
+    const uint32_t i = warp->found;
+    if (i < kSettleLater) {
+        warp->later[i] = warp->tag + at;
+        warp->found = i + 1;
+    } else {
+        atomicOr(fail, fail_bit);
+    }
+}
+
+// the largest d <= most with ok(d), by a warp: 32 probes a round; ok(lo) holds, and ok is true up to that d
+template <typename F>
+__device__ __forceinline__ uint32_t warp_last(uint32_t lo, uint32_t most, F ok) {
+    uint32_t hi = most + 1;                               // the first that may not be
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32, d = lo + ((threadIdx.x & 31u) + 1) * step;
+        const uint32_t c = uint32_t(__popc(__ballot_sync(0xFFFFFFFFu, d < hi && ok(d))));
+        hi = min(hi, lo + (c + 1) * step);
+        lo += c * step;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ void or_diff(uint64_t &acc, uint64_t a, uint64_t b) { acc |= a ^ b; }
+template <int HB>
+__device__ __forceinline__ void or_diff(KeyWide<HB> &acc, KeyWide<HB> a, KeyWide<HB> b) {
+    acc.lo |= a.lo ^ b.lo;
+    acc.hi |= a.hi ^ b.hi;
+}
+// the digits in which any lane's bits are set
+__device__ __forceinline__ uint32_t diff_digits(uint64_t d) {
+    const uint32_t w[2] = {__reduce_or_sync(0xFFFFFFFFu, uint32_t(d)), __reduce_or_sync(0xFFFFFFFFu, uint32_t(d >> 32))};
+    uint32_t m = 0;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) m |= ((w[p / 4] >> (p % 4 * 8)) & 0xFFu) ? 1u << p : 0u;
+    return m;
+}
+template <int HB>
+__device__ __forceinline__ uint32_t diff_digits(KeyWide<HB> d) { return diff_digits(d.lo) | (diff_digits(d.hi) << 8); }
+
+// One warp sorts the group that has an inversion at key `at`, if it is longer than its chunk's view and no other
+// warp has taken it up: a stable pass per digit below the prefix that is not the same in all, ranked by matching
+// digits, between the group's place and the same place in the free arrays (a key's place always holds a key of
+// the group, as the neighbours' reads want it).  A pass counts the next one's digits as it goes.
+template <int MODE, bool HAS_VAL, typename U>
+__device__ __noinline__ void settle_long(U *keys, uint64_t *vals, uint64_t at, uint64_t n, U mask, bool desc, SettleWarp<U> *warp,
+                                         const SettleLong<U> &w, uint32_t *fail, uint32_t fail_bit) {
+    using S = SettleShape<U>;
+    constexpr int B = sizeof(U) == 8 && !HAS_VAL ? 8 : 4;     // loads of a lane in flight
+    static_assert(sizeof(warp->key) >= 2 * kBuckets * 4, "the offsets and the next counts fit the view's memory");
+    const int lane = int(threadIdx.x & 31u);
+    const uint32_t limit = uint32_t(w.limit);
+    const U ref = settle_order<MODE>(keys[at], desc);
+    auto same = [&](uint64_t i) { return same_masked(settle_order<MODE>(keys[i], desc), ref, mask); };
+    const uint32_t back = warp_last(1, uint32_t(at < limit ? at : limit), [&](uint32_t d) { return same(at - d); });
+    const uint32_t on = warp_last(0, uint32_t(n - 1 - at < limit ? n - 1 - at : limit), [&](uint32_t d) { return same(at + d); });
+    const uint32_t len = back + on + 1;
+    const uint64_t s = at - back, c0 = s / S::kChunk * S::kChunk;
+    if (s + len < c0 + S::kView || c0 + S::kView >= n) return;      // settle_wide's
+    int mine = -1;
+    if (lane == 0 && len <= limit) mine = settle_take(w, s + w.tag + 1u);
+    mine = __shfl_sync(0xFFFFFFFFu, mine, 0);
+    if (mine < 0 && lane == 0) atomicOr(fail, fail_bit);
+    if (mine <= 0) return;
+    uint32_t *off = reinterpret_cast<uint32_t *>(warp->key), *cnt = off + kBuckets;
+    U *src = keys + s, *dst = w.free_keys + s;
+    uint64_t *src_v = vals, *dst_v = vals;
+    if constexpr (HAS_VAL) {
+        src_v = vals + s;
+        dst_v = w.free_vals + s;
+    }
+    U diff{};
+    for (uint32_t x0 = 0; x0 < len; x0 += 32 * B) {
+        U k[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) k[q] = src[min(x0 + uint32_t(q * 32 + lane), len - 1)];
+#pragma unroll
+        for (int q = 0; q < B; ++q) or_diff(diff, settle_order<MODE>(k[q], desc), ref);
+    }
+    const uint32_t digits = diff_digits(diff) & w.digits;
+    for (int i = lane; i < kBuckets; i += 32) cnt[i] = 0;
+    __syncwarp();
+    if (digits) {
+        const int p = __ffs(digits) - 1;
+        for (uint32_t x0 = 0; x0 < len; x0 += 32 * B) {
+            U k[B];
+#pragma unroll
+            for (int q = 0; q < B; ++q) k[q] = src[min(x0 + uint32_t(q * 32 + lane), len - 1)];
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+                if (x0 + uint32_t(q * 32 + lane) < len) atomicAdd(cnt + digit_of(settle_order<MODE>(k[q], desc), p), 1u);
+        }
+    }
+    for (uint32_t m = digits; m; m &= m - 1) {
+        const int p = __ffs(m) - 1, next = (m & (m - 1)) ? __ffs(m & (m - 1)) - 1 : -1;
+        __syncwarp();
+        uint32_t sum = 0;
+#pragma unroll
+        for (int i = 0; i < kBuckets / 32; ++i) sum += cnt[lane * (kBuckets / 32) + i];
+        uint32_t to0 = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, to0, o);
+            if (lane >= o) to0 += y;
+        }
+        to0 -= sum;
+#pragma unroll
+        for (int i = 0; i < kBuckets / 32; ++i) {
+            off[lane * (kBuckets / 32) + i] = to0;
+            to0 += cnt[lane * (kBuckets / 32) + i];
+            cnt[lane * (kBuckets / 32) + i] = 0;
+        }
+        __syncwarp();
+        for (uint32_t x0 = 0; x0 < len; x0 += 32 * B) {
+            U k[B];
+            uint64_t v[HAS_VAL ? B : 1];
+#pragma unroll
+            for (int q = 0; q < B; ++q) {
+                const uint32_t x = min(x0 + uint32_t(q * 32 + lane), len - 1);
+                k[q] = src[x];
+                if constexpr (HAS_VAL) v[q] = src_v[x];
+            }
+#pragma unroll
+            for (int q = 0; q < B; ++q) {
+                const bool in = x0 + uint32_t(q * 32 + lane) < len;
+                const U b = settle_order<MODE>(k[q], desc);
+                const uint32_t d = in ? digit_of(b, p) : uint32_t(kBuckets);
+                const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d), before = uint32_t(__popc(peers & ((1u << lane) - 1u)));
+                const uint32_t to = in ? off[d] + before : len;
+                __syncwarp();
+                if (in && before == 0) off[d] += uint32_t(__popc(peers));
+                __syncwarp();
+                if (to < len) {
+                    dst[to] = k[q];
+                    if constexpr (HAS_VAL) dst_v[to] = v[q];
+                }
+                if (in && next >= 0) atomicAdd(cnt + digit_of(b, next), 1u);
+            }
+        }
+        U *t = src;
+        src = dst;
+        dst = t;
+        uint64_t *tv = src_v;
+        src_v = dst_v;
+        dst_v = tv;
+    }
+    __syncwarp();
+    if (src != keys + s) {
+#pragma unroll 4
+        for (uint32_t x = uint32_t(lane); x < len; x += 32) {
+            dst[x] = src[x];
+            if constexpr (HAS_VAL) dst_v[x] = src_v[x];
+        }
+    }
+    __syncwarp();                                         // the warp's shared memory is free again
+}
+
 // one warp settles the groups that start in the chunk at c0, in shared memory
 template <int MODE, bool HAS_VAL, typename S, typename U>
-__device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, U *key,
-                                         uint32_t *hw, uint32_t *vw, uint32_t *fail, uint32_t fail_bit) {
+__device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, SettleWarp<U> *warp,
+                                         uint32_t *fail, uint32_t fail_bit) {
     constexpr int WORDS = S::kWords;
+    U *key = warp->key;
+    uint32_t *hw = warp->head, *vw = warp->inv;
     const int lane = int(threadIdx.x & 31u);
     const int view = int(n - c0 < uint64_t(S::kView) ? n - c0 : uint64_t(S::kView));
     for (int x = lane; x < view; x += 32) key[x] = keys[c0 + x];
@@ -308,7 +520,7 @@ __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, u
         int e = bit_at_or_above(hw, x + 1, WORDS);
         if (e >= view) {
             if (c0 + uint64_t(view) < n) {                // it runs on past the view
-                if (lane == 0) atomicOr(fail, fail_bit);
+                if (lane == 0) settle_later(warp, c0 + uint64_t(x), fail, fail_bit);
                 break;
             }
             e = view;
@@ -333,10 +545,11 @@ __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, u
     __syncwarp();                                         // the warp's shared memory is free again
 }
 
-// one warp settles the groups that start in the chunk at c0 (raising fail_bit in *fail where it cannot)
+// one warp settles the groups that start in the chunk at c0, and keeps what it meets of long groups for later (a
+// call of settle_long from here would cost the loop around it registers)
 template <int MODE, bool HAS_VAL, typename S, typename U>
-__device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, U *key_s,
-                                             uint32_t *hw, uint32_t *vw, uint32_t *fail, uint32_t fail_bit) {
+__device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, SettleWarp<U> *warp,
+                                             uint32_t *fail, uint32_t fail_bit) {
     constexpr int ITEMS = S::kItems, C = S::kChunk;
     // v holds the keys as they are where ordering them takes an exclusive-or, else as the sort orders them:
     // a key that moves is then fetched again from where it came (as a pointer is)
@@ -387,13 +600,13 @@ __device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c
     const uint32_t out = lane == 31 ? ~below & 0xFFu : 0u;
     const uint32_t bad_in = vb & in;
     if (__any_sync(0xFFFFFFFFu, bad_in != 0)) {
-        // settled by the chunk before, if it holds the start and sees the inversion
-        bool lost = bad_in && lane * ITEMS + 31 - __clz(bad_in) >= S::kReach;
+        // met by the chunk before too, if it holds the start and has the inversion in its view
+        bool left = bad_in && lane * ITEMS + 31 - __clz(bad_in) >= S::kView - C;
         if (bad_in && c0 > uint64_t(C)) {
             const U a = settle_order<MODE>(keys[c0 - C - 1], desc), b = settle_order<MODE>(keys[c0 - 1], desc);
-            lost |= same_masked(a, b, mask);
+            left |= same_masked(a, b, mask);
         }
-        if (lost) atomicOr(fail, fail_bit);
+        if (left) settle_later(warp, c0 + uint64_t(lane * ITEMS + 31 - __clz(bad_in)), fail, fail_bit);
     }
     const uint32_t pass = ~hb & ~in & ~out & 0xFFu;          // keys that may pass the one before them
     bool wide = open;
@@ -473,8 +686,7 @@ __device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c
                 if ((moved >> j) & 1u) dst[j] = v[j];
         }
     }
-    if (wide)
-        settle_wide<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc, key_s, hw, vw, fail, fail_bit);
+    if (wide) settle_wide<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc, warp, fail, fail_bit);
 }
 
 template <typename U, int MODE, bool HAS_VAL>
@@ -487,39 +699,63 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
     after_previous();
     const uint32_t k = ctrl->prefix_passes, low = ctrl->prefix_low, survive = ctrl->survive;
     if (k == 0 || ctrl->abort) return;
-    __shared__ __align__(16) U keys_s[S::kWarps][S::kView];
-    __shared__ uint32_t words_s[S::kWarps][2][S::kWords];
+    __shared__ SettleWarp<U> warps[S::kWarps];
     __shared__ uint32_t last;
     const int tid = threadIdx.x, warp = tid >> 5;
     bool bad = !prefix_in_range<KeyTraits<U>::kDigits>(k, low, survive);
-    const PassPlan end = ctrl->plan[bad ? 0u : k - 1];
+    const PassPlan &end = ctrl->plan[bad ? 0u : k - 1];
     U *keys = static_cast<U *>(sort_array(arrs, end.dst_keys, HAS_VAL ? kArrKeysA : kArrBuf, &bad));
     uint64_t *vals = static_cast<uint64_t *>(sort_array(arrs, end.dst_vals, kArrBuf, &bad));
     if (bad || !keys || (HAS_VAL && !vals)) {       // a damaged control block
         if (tid == 0) atomicOr(&ctrl->error, kDevFault);
         return;
     }
+    if ((tid & 31) == 0) {
+        warps[warp].found = 0;
+        warps[warp].tag = 0;
+    }
+    __syncwarp();
     // the prefix passes' look-back words, cleared for the plain passes that a failure calls for
     for (uint64_t i = uint64_t(blockIdx.x) * THREADS + tid; i < uint64_t(k) * status_bytes / 16; i += uint64_t(gridDim.x) * THREADS)
         reinterpret_cast<uint4 *>(status)[i] = make_uint4(0, 0, 0, 0);
     const U mask = prefix_mask<U>(low);
-    const uint64_t chunks = (n + C - 1) / C, stride = uint64_t(gridDim.x) * S::kWarps;
-    uint32_t seen = 0;
-    for (uint64_t c = uint64_t(blockIdx.x) * S::kWarps + warp; c < chunks; c += stride) {
-        // the failure flag is one word for the whole grid: looked at now and then
-        if ((++seen & 15u) == 0 && ld_relaxed(&ctrl->settle_fail)) break;
-        settle_chunk<MODE, HAS_VAL, S>(keys, vals, c * C, n, mask, desc != 0, keys_s[warp], words_s[warp][0], words_s[warp][1],
-                                       &ctrl->settle_fail, 1u);
+    const uint64_t stride = uint64_t(gridDim.x) * S::kCtaKeys;
+    for (uint64_t c0 = uint64_t(blockIdx.x) * S::kCtaKeys + uint32_t(warp * C); c0 < n; c0 += stride)
+        settle_chunk<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc != 0, &warps[warp], &ctrl->settle_fail, 1u);
+    __syncwarp();
+    if (warps[warp].found && !__any_sync(0xFFFFFFFFu, ld_relaxed(&ctrl->settle_fail) != 0)) {
+        // the array that is free: what the last pass read from or could have, the copy forms' buffer or the in-place
+        // forms' other array; the table of long groups lies where the last digit's look-back words do, which are
+        // clear (a prefix leaves two digits out)
+        const uint32_t free = (HAS_VAL ? end.dst_vals : end.dst_keys) == kArrBuf ? (pa.inplace ? kArrIn : kArrOut) : kArrBuf;
+        void *arr = sort_array(arrs, free, kArrBuf, &bad);
+        SettleLong<U> w;
+        w.free_keys = HAS_VAL ? static_cast<U *>(sort_array(arrs, end.dst_keys == kArrKeysA ? kArrKeysB : kArrKeysA, kArrKeysA, &bad))
+                              : static_cast<U *>(arr);
+        w.free_vals = static_cast<uint64_t *>(arr);
+        w.taken = reinterpret_cast<unsigned long long *>(status + (KeyTraits<U>::kDigits - 1) * status_bytes);
+        w.tag = 0;
+        w.limit = settle_limit(n);
+        w.room = uint32_t(status_bytes / 8 < kTakenRoom ? status_bytes / 8 : kTakenRoom);
+        w.digits = survive & ((1u << low) - 1u);
+        bad = __any_sync(0xFFFFFFFFu, bad);
+        for (uint32_t i = 0; i < warps[warp].found && !bad; ++i)
+            settle_long<MODE, HAS_VAL>(keys, vals, warps[warp].later[i], n, mask, desc != 0, &warps[warp], w, &ctrl->settle_fail, 1u);
     }
     __threadfence();
     __syncthreads();
     if (tid == 0) last = atomicAdd(&ctrl->settle_done, 1u) == gridDim.x - 1 ? 1u : 0u;
     __syncthreads();
-    if (!last || tid != 0 || !ld_relaxed(&ctrl->settle_fail)) return;
+    if (!last || !ld_relaxed(&ctrl->settle_fail)) return;
     // a group was too long to settle: the plain passes, over every digit, from where the data stand
-    const uint32_t cur = HAS_VAL ? end.dst_vals : end.dst_keys;
+    // (the table of long groups is cleared for them)
+    for (uint64_t i = tid; i < status_bytes / 8 && i < kTakenRoom; i += THREADS)
+        reinterpret_cast<unsigned long long *>(status + (KeyTraits<U>::kDigits - 1) * status_bytes)[i] = 0;
+    if (tid != 0) return;
+    const uint32_t digits = ctrl->survive & ((1u << KeyTraits<U>::kDigits) - 1u);
     uint32_t curk = end.dst_keys;
-    const uint32_t done = plan_chain(ctrl, pa, ctrl->hot, survive, !pa.inplace, kPrefixSlots, cur, curk, false, false);
+    const uint32_t done = plan_chain(ctrl, pa, ctrl->hot, digits, !pa.inplace, kPrefixSlots, HAS_VAL ? end.dst_vals : end.dst_keys,
+                                     curk, false, false);
     plan_copy(ctrl, pa, done, false);
 }
 

@@ -192,7 +192,7 @@ cudaError_t launch_segmented_mode_t(const Resolved &r, const SegArgs &args, cons
         if constexpr (KeyTraits<U>::kDigits >= 8) {
             if (phase) {
                 LaunchTimer t(s, RSBD8G_KERNEL_SETTLE, uint32_t(sizeof(U)), 0, a.nsegs);
-                e = seg_launch<U>(k_seg_settle<U, MODE>, uint32_t(seg_settle_setup<U, MODE>(dev) * sms), SettleShape<U>::kThreads, 0, s, a, out);
+                e = seg_launch<U>(k_seg_settle<U, MODE>, uint32_t(seg_settle_setup<U, MODE>(dev) * sms), SettleShape<U>::kThreads, 0, s, a, out, buf);
                 if (e != cudaSuccess) return e;
             }
         }

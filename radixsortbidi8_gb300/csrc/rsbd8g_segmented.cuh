@@ -60,6 +60,8 @@ struct SegArgs {
     const uint8_t *seg_dir;
     uint32_t rev_ok;
     uint32_t prefix_ok;       // 8- and 16-byte keys: segments may be sorted by a prefix and settled
+    uint32_t *status;         // look-back words of the tiles, of status_bytes bytes (more than the tiles take)
+    uint64_t status_bytes;
 };
 
 // the digit complement (descending sorts) and the effective isrevorder of segment `seg`
@@ -331,6 +333,13 @@ static __global__ void __launch_bounds__(256) k_seg_plan(SegArgs a, int passes) 
     if (t == 0 && all0) atomicOr(&c->pass_mask[0], all0);
 }
 
+// the table of long groups of k_seg_settle (SettleWarp::taken): behind the tiles' look-back words; its entries
+__device__ __forceinline__ uint32_t seg_taken(const SegArgs &a, unsigned long long **taken) {
+    const uint64_t used = uint64_t(a.ctrl->ntiles) * kBuckets * 4u;
+    *taken = reinterpret_cast<unsigned long long *>(reinterpret_cast<unsigned char *>(a.status) + used);
+    return used < a.status_bytes ? uint32_t(min((a.status_bytes - used) / 8u, uint64_t(kTakenRoom))) : 0u;
+}
+
 // The plan of 8- and 16-byte keys: beside k_seg_plan's work, samples of the segment decide whether it is
 // sorted by a prefix of its digits (a round of 256 keys for every 2^15 keys, 17 at most: a segment of over
 // 2^20 keys is not sorted by a prefix).  One CTA per segment.
@@ -345,6 +354,11 @@ __global__ void __launch_bounds__(256) k_seg_plan_wide(SegArgs a, const U *__res
     __shared__ __align__(16) U sample[256];
     const uint32_t nl = c->nlarge;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (a.prefix_ok && blockIdx.x == 0) {                // k_seg_settle's table is empty
+        unsigned long long *taken;
+        const uint32_t room = seg_taken(a, &taken);
+        for (uint32_t i = t; i < room; i += 256u) taken[i] = 0;
+    }
     uint32_t all0 = 0;
     for (uint32_t idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         const uint32_t seg = a.large_seg[idx];
@@ -397,17 +411,18 @@ static __global__ void __launch_bounds__(256) k_seg_clear(SegArgs a, int pass, i
 // the settle step of the segments sorted by a prefix, in place in their output: warps take quarters of
 // the large segments' tiles in turn (a quarter: the chunks that start in it)
 template <typename U, int MODE>
-__global__ void __launch_bounds__(SettleShape<U>::kThreads, 4) k_seg_settle(SegArgs a, U *__restrict__ out) {
+__global__ void __launch_bounds__(SettleShape<U>::kThreads, 4) k_seg_settle(SegArgs a, U *out, U *buf) {
     using S = SettleShape<U>;
     next_may_start();
     after_previous();
     SegControl *c = a.ctrl;
     if (c->abort) return;
-    __shared__ __align__(16) U keys_s[S::kWarps][S::kView];
-    __shared__ uint32_t words_s[S::kWarps][2][S::kWords];
+    __shared__ SettleWarp<U> warps[S::kWarps];
     const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
     const uint64_t units = uint64_t(c->ntiles) * 4u, stride = uint64_t(gridDim.x) * S::kWarps;
     const uint32_t part = a.tile / 4u;
+    uint64_t *const none = nullptr;
+    if (lane == 0) warps[warp].found = 0;
     for (uint64_t u = uint64_t(blockIdx.x) * S::kWarps + warp; u < units; u += stride) {
         const uint32_t gt = uint32_t(u / 4u), idx = a.tile_seg[gt], how = a.seg_mask[idx];
         if (!(how & kSegPrefix)) continue;
@@ -419,10 +434,29 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, 4) k_seg_settle(SegA
         U *keys = seg_ptr(a, a.ptr_out, out, seg);
         const U mask = prefix_mask<U>((how >> 16) & 31u);
         const bool desc = seg_dmask(a, seg) != 0;
-        for (uint64_t x = (k0 + S::kChunk - 1) / S::kChunk; x * S::kChunk < k1; ++x)
-            settle_chunk<MODE, false, S>(keys, static_cast<uint64_t *>(nullptr), x * S::kChunk, n, mask, desc, keys_s[warp],
-                                         words_s[warp][0], words_s[warp][1], a.seg_mask + idx, kSegFail);
+        if (lane == 0) warps[warp].tag = uint64_t(idx) << 32;
         __syncwarp();
+        for (uint64_t x = (k0 + S::kChunk - 1) / S::kChunk; x * S::kChunk < k1; ++x)
+            settle_chunk<MODE, false, S>(keys, none, x * S::kChunk, n, mask, desc, &warps[warp], a.seg_mask + idx, kSegFail);
+        __syncwarp();
+        if (lane == 0 && (ld_relaxed(a.seg_mask + idx) & kSegFail)) atomicOr(&c->pass_mask[1], how & 0xFFFFu);
+    }
+    __syncwarp();
+    for (uint32_t i = 0; i < warps[warp].found; ++i) {
+        const uint32_t idx = uint32_t(warps[warp].later[i] >> 32), seg = a.large_seg[idx];
+        const uint32_t how = __shfl_sync(0xFFFFFFFFu, ld_relaxed(a.seg_mask + idx), 0);
+        if (how & kSegFail) continue;
+        const uint64_t n = seg_len(a.offsets, seg);
+        const uint32_t low = (how >> 16) & 31u;
+        SettleLong<U> w;
+        w.free_keys = seg_ptr(a, a.ptr_buf, buf, seg);
+        w.free_vals = none;
+        w.room = seg_taken(a, &w.taken);
+        w.tag = uint64_t(idx) << 32;
+        w.limit = settle_limit(n);
+        w.digits = how & 0xFFFFu & ((1u << low) - 1u);
+        settle_long<MODE, false>(seg_ptr(a, a.ptr_out, out, seg), none, warps[warp].later[i] & 0xFFFFFFFFu, n, prefix_mask<U>(low),
+                                 seg_dmask(a, seg) != 0, &warps[warp], w, a.seg_mask + idx, kSegFail);
         if (lane == 0 && (ld_relaxed(a.seg_mask + idx) & kSegFail)) atomicOr(&c->pass_mask[1], how & 0xFFFFu);
     }
 }

@@ -125,6 +125,8 @@ static rsbd8g_status segmented_common(const rsbd8g_desc *desc, size_t total, siz
     a.seg_hist = reinterpret_cast<uint32_t *>(sc + L.seg_hist);
     a.seg_mask = reinterpret_cast<uint32_t *>(sc + L.seg_mask);
     a.tile_seg = reinterpret_cast<uint32_t *>(sc + L.tile_seg);
+    a.status = reinterpret_cast<uint32_t *>(sc + L.status);
+    a.status_bytes = L.status_bytes;
     a.ptr_in = in_ptrs;
     a.ptr_out = out_ptrs;
     a.ptr_buf = buf_ptrs;

@@ -101,3 +101,161 @@ def test_segments_of_one_value_are_copied(kt, direction):
     got = s.run().cpu().numpy().view(kt)
     for b, e in zip(offs[:-1], offs[1:]):
         assert same_bits(got[b:e], O.sortcopy(a[b:e], "nativeabs", direction))
+
+
+def plan_of(scratch):
+    """what the plain sort did, from its control block (Control of rsbd8g_device.cuh, at the scratch's start)"""
+    import torch
+    torch.cuda.synchronize()
+    w = scratch[:160].cpu().numpy().view(np.uint32)
+    return dict(error=int(w[0]), low=int(w[31]), passes=int(w[32]), failed=int(w[33]))
+
+
+DRAWS = 160 * 1024                  # of one round, up to 160 histogram CTAs
+CROWDS = [(3000, 0), (4000, 0), (30000, 1)]          # the last is too long to settle
+
+
+@pytest.mark.parametrize("size,failed", CROWDS)
+@pytest.mark.parametrize("form", ["copy", "inplace", "tobuffer"])
+def test_a_crowd_that_no_sample_saw(size, failed, form):
+    """out-of-order groups longer than a warp's view: up to settle_limit (4096 of 2^21 keys) they are settled, in
+    the array that the passes left free; beyond it the plain passes run"""
+    import torch
+    import radixsortbidi8_gb300 as rs
+    n = (1 << 21) + 77
+    a = with_crowd(n, size, DRAWS).view(np.int64)
+    x = torch.from_numpy(a.copy()).cuda()
+    y, buf = torch.empty_like(x), torch.empty_like(x)
+    for direction in ("ascfwdorder", "dscfwdorder"):
+        x.copy_(torch.from_numpy(a))
+        scratch = torch.empty(rs.scratch_bytes(np.int64, n, direction, "native"), dtype=torch.uint8, device="cuda")
+        if form == "copy":
+            rs.radixsortcopynoalloc(x, y, buf, scratch, direction, "native", key_dtype=np.int64)
+        else:
+            rs.radixsortnoalloc(x, buf, scratch, form == "tobuffer", direction, "native", key_dtype=np.int64)
+        p = plan_of(scratch)
+        assert p["passes"] > 0 and p["failed"] == failed and p["error"] == 0, p
+        got = (y if form == "copy" else x if form == "inplace" else buf).cpu().numpy()
+        assert same_bits(got, O.sortcopy(a, "native", direction))
+        if form == "copy":
+            assert same_bits(x.cpu().numpy(), a)          # the copy form leaves its input alone
+
+
+CHUNK, VIEW = 248, 472              # SettleShape::kChunk, kView
+
+
+def crowds_of_every_length(n, lengths):
+    """a crowd of each length, spread over the key range; and where each starts and ends in the sorted array"""
+    a = S.uniform_bits(21, n, np.uint64)
+    at, o = unseen(n, int(np.sum(lengths)), DRAWS, 22), 0
+    tops = np.sort(S.uniform_bits(23, len(lengths), np.uint64)) & np.uint64(0xFFFFFFFFFF000000)
+    for top, m in zip(tops, lengths):
+        p = at[o:o + m]
+        a[p] = top | (a[p] & np.uint64(0xFFFFFF))
+        o += m
+    srt = np.sort(a) >> np.uint64(24)
+    return a, np.searchsorted(srt, tops >> np.uint64(24)), np.searchsorted(srt, tops >> np.uint64(24), side="right")
+
+
+def test_crowds_about_the_view():
+    """crowds that end before, at and after the end of the view of the chunk they start in, and of the next"""
+    import torch
+    import radixsortbidi8_gb300 as rs
+    n = 1 << 22
+    a, b, e = crowds_of_every_length(n, np.tile(np.arange(200, 760), 2))
+    past = e - (b // CHUNK * CHUNK + VIEW)
+    assert {-1, 0, 1} <= set(past.tolist())
+    x = torch.from_numpy(a.view(np.int64)).cuda()
+    y, buf = torch.empty_like(x), torch.empty_like(x)
+    scratch = torch.empty(rs.scratch_bytes(np.uint64, n), dtype=torch.uint8, device="cuda")
+    rs.radixsortcopynoalloc(x, y, buf, scratch, key_dtype=np.uint64)
+    p = plan_of(scratch)
+    assert p["passes"] > 0 and p["failed"] == 0 and p["error"] == 0, p
+    assert same_bits(y.cpu().numpy().view(np.uint64), np.sort(a))
+
+
+@pytest.mark.parametrize("size,failed", CROWDS)
+@pytest.mark.parametrize("mode,direction", [("nativeabs", "ascrevorder"), ("nativeabs", "dscrevorder"), ("native", "ascrevorder")])
+def test_a_crowd_of_floats_with_ties(size, failed, mode, direction):
+    """float orders: the crowd's values come eight times each, and under nativeabs with both signs (reversed ties)"""
+    import torch
+    import radixsortbidi8_gb300 as rs
+    n = (1 << 21) + 77
+    a = with_crowd(n, size, DRAWS) & np.uint64((1 << 63) - 1)
+    at = np.flatnonzero(a >> np.uint64(24) == 0x77777777)
+    a[at] = a[at[np.arange(at.size) // 8 * 8]] ^ ((S.uniform_bits(6, at.size, np.uint64) & np.uint64(1)) << np.uint64(63) if mode == "nativeabs"
+                                                  else np.uint64(0))
+    x = torch.from_numpy(a.view(np.int64)).cuda()
+    y, buf = torch.empty_like(x), torch.empty_like(x)
+    scratch = torch.empty(rs.scratch_bytes(np.float64, n, direction, mode), dtype=torch.uint8, device="cuda")
+    rs.radixsortcopynoalloc(x, y, buf, scratch, direction, mode, key_dtype=np.float64)
+    p = plan_of(scratch)
+    assert p["passes"] > 0 and p["failed"] == failed and p["error"] == 0, p
+    assert same_bits(y.cpu().numpy().view(np.float64), O.sortcopy(a.view(np.float64), mode, direction))
+
+
+@pytest.mark.parametrize("size,failed", CROWDS)
+@pytest.mark.parametrize("direction", ["ascfwdorder", "dscrevorder"])
+def test_a_crowd_of_pointers(size, failed, direction):
+    import torch
+    import radixsortbidi8_gb300 as rs
+    from radixsortbidi8_gb300 import api
+    n = (1 << 21) + 77
+    key = with_crowd(n, size, 640 * 512)                  # up to 640 CTAs of 512 gather
+    at = np.flatnonzero(key >> np.uint64(24) == 0x77777777)
+    key[at] = key[at[np.arange(at.size) // 4 * 4]]        # ties
+    rec = torch.zeros((n, 2), dtype=torch.int64, device="cuda")
+    rec[:, 1] = torch.from_numpy(key.view(np.int64)).cuda()
+    ptr = rec.data_ptr() + 16 * torch.arange(n, dtype=torch.int64, device="cuda")
+    out, buf = torch.empty_like(ptr), torch.empty_like(ptr)
+    scratch = torch.empty(rs.scratch_bytes(np.uint64, n, direction, "native", indirection=api.MEMBER, offset1=8), dtype=torch.uint8, device="cuda")
+    rs.radixsortcopynoalloc_member(ptr, out, buf, scratch, np.uint64, 8, direction, "native")
+    p = plan_of(scratch)
+    assert p["passes"] > 0 and p["failed"] == failed and p["error"] == 0, p
+    k = key if direction == "ascfwdorder" else ~key
+    order = np.argsort(k, kind="stable") if direction == "ascfwdorder" else n - 1 - np.argsort(k[::-1], kind="stable")
+    assert np.array_equal(out.cpu().numpy(), rec.data_ptr() + 16 * order)
+
+
+@pytest.mark.parametrize("size,failed", [(1500, 0), (2000, 0), (30000, 1)])
+@pytest.mark.parametrize("kind,mode,direction", [("u128", "native", "dscfwdorder"), ("f128", "native", "ascrevorder"), ("x87", "nativeabs", "ascrevorder")])
+def test_a_crowd_of_16_byte_keys(size, failed, kind, mode, direction):
+    """(settle_limit is 2048 of 2^20 keys)"""
+    import torch
+    import radixsortbidi8_gb300 as rs
+    n = 1 << 20
+    hi = with_crowd(n, size, DRAWS) & np.uint64((1 << 63) - 1)
+    lo = S.uniform_bits(8, n, np.uint64)
+    at = np.flatnonzero(hi >> np.uint64(24) == 0x77777777)
+    if kind == "x87":                 # 64-bit significands of one exponent: the crowd in the low word, signs mixed
+        w = np.stack([hi, np.uint64(0x3FFF) | ((lo & np.uint64(1)) << np.uint64(15))], axis=1)
+    else:
+        w = np.stack([lo, hi], axis=1)
+    w[at] = w[at[np.arange(at.size) // 2 * 2]]            # ties
+    x = torch.from_numpy(w.view(np.int64).reshape(-1)).cuda()
+    y, buf = torch.empty_like(x), torch.empty_like(x)
+    scratch = torch.empty(rs.scratch_bytes(kind, n, direction, mode), dtype=torch.uint8, device="cuda")
+    rs.radixsortcopynoalloc(x, y, buf, scratch, direction, mode, key_dtype=kind)
+    p = plan_of(scratch)
+    assert p["passes"] > 0 and p["failed"] == failed and p["error"] == 0, p
+    want = O.sortcopy_wide(w, kind, mode, direction)
+    assert np.array_equal(y.cpu().numpy().view(np.uint64).reshape(n, 2), np.asarray(want).reshape(n, 2))
+
+
+@pytest.mark.parametrize("kt,mode,direction", [(np.int64, "native", "ascfwdorder"), (np.float64, "nativeabs", "dscrevorder"),
+                                               (np.float64, "native", "ascrevorder")], ids=str)
+@pytest.mark.parametrize("size,failed", [(1500, 0), (30000, 1)])
+def test_a_crowd_in_a_batch(kt, mode, direction, size, failed):
+    """(settle_limit is 2048 of 600,000 keys); the ties of a failed segment turn once, not twice"""
+    segs = [segment(600011, size, i, 3 + i) & np.uint64((1 << 63) - 1) for i in range(4)]
+    for sg in segs:
+        at = np.flatnonzero(sg >> np.uint64(24) == 0x77777777)
+        sg[at] = sg[at[np.arange(at.size) // 4 * 4]]
+        if mode == "nativeabs":
+            sg[1::2] |= np.uint64(1 << 63)
+    a, offs, s = sorter(segs, kt, direction, mode)
+    got = s.run().cpu().numpy().view(kt)
+    for b, e in zip(offs[:-1], offs[1:]):
+        assert same_bits(got[b:e], O.sortcopy(a[b:e].view(kt), mode, direction))
+    first, second = seg_passes(s)
+    assert first and not first & 1 and (second != 0) == bool(failed), (first, second)
