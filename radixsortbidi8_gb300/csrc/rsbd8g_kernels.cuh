@@ -108,8 +108,9 @@ __device__ __forceinline__ void plan_body(Control *__restrict__ ctrl, const unsi
     ctrl->stall_tile = a.stall_tile;
     ctrl->prefetch = a.prefetch;
     uint32_t curk = kArrKeysA, low = 0;
-    const uint32_t k = a.prefix_ok ? prefix_choose(pairs, survive, n, uint64_t(prefix_rounds(n)) * gridDim.x * blockDim.x * (blockDim.x - 1u) / 2u,
-                                                     &low) : 0u;
+    const uint32_t ctas = gridDim.x, size = a.indirect ? prefix_size<kSampleGather, kSampleGather>(n, ctas)
+                                                       : prefix_size<kSampleLeast, kSampleDirect>(n, ctas);
+    const uint32_t k = a.prefix_ok ? prefix_choose(pairs, survive, n, prefix_rounds(n, ctas, size) * prefix_pairs(ctas, size), &low) : 0u;
     ctrl->prefix_passes = k;
     ctrl->prefix_low = low;
     if (k) {
@@ -200,9 +201,12 @@ __global__ void __launch_bounds__(THREADS) k_histogram(const U *__restrict__ key
     constexpr int C = hist_lane_copies<P>();
     constexpr int V = 16 / int(sizeof(U));
     extern __shared__ __align__(16) uint32_t shl[];
+    // the samples of wide keys are drawn now and sorted when the counts are on their way (2^28 int64 keys: 562 us with
+    // the samples ahead of the counting, 543 so)
+    U draw{};
+    auto filtered = [&](uint64_t i) { return filter_key<MODE>(keys[i]); };
     if constexpr (P >= 8) {
-        if (pa.prefix_ok)
-            prefix_sample_cta<U, THREADS>(reinterpret_cast<U *>(shl), n, ctrl, [&](uint64_t i) { return filter_key<MODE>(keys[i]); });
+        if (pa.prefix_ok) draw = prefix_draw<U, kSampleLeast, kSampleDirect>(n, filtered);
     }
     for (int i = threadIdx.x; i < C * P * kBuckets; i += THREADS) shl[i] = 0;
     __syncthreads();
@@ -248,6 +252,12 @@ __global__ void __launch_bounds__(THREADS) k_histogram(const U *__restrict__ key
         for (int c = 0; c < C; ++c) t += shl[i * C + ((c + i) & (C - 1))];
         if (t) atomicAdd(ghist + i, (unsigned long long)t);
     }
+    if constexpr (P >= 8) {
+        if (pa.prefix_ok) {
+            __syncthreads();                 // the counters have been read: the sample takes their place
+            prefix_sample_cta<U, THREADS, kSampleLeast, kSampleDirect>(reinterpret_cast<U *>(shl), n, ctrl, draw, filtered);
+        }
+    }
     plan_if_last<THREADS>(ctrl, ghist, bstart, n, pa);
 }
 
@@ -259,6 +269,15 @@ __device__ __noinline__ U gathered_key(const uint64_t *ptrs, uint64_t i, int64_t
     const unsigned char *obj = reinterpret_cast<const unsigned char *>(ptrs[i]) + off1;
     if (level == 2) obj = load_ptr(obj) + off2;
     return load_member<U>(obj);
+}
+
+// the samples of an indirect sort, ahead of its loop (behind it they took 3 to 8 us more; a call: in line, they took
+// registers from the loop)
+template <typename U, int MODE, int THREADS>
+__device__ __noinline__ void gather_sample(U *s, const uint64_t *ptrs, uint64_t n, int64_t off1, int64_t off2, int level, const U *keys_in,
+                                           Control *ctrl) {
+    auto key = [=](uint64_t i) { return filter_key<MODE>(gathered_key<U>(ptrs, i, off1, off2, level, keys_in)); };
+    prefix_sample_cta<U, THREADS, kSampleGather, kSampleGather>(s, n, ctrl, U{}, key);
 }
 
 // indirect form: gather the key through each object pointer (level 1: at off1; level 2: behind the
@@ -274,10 +293,10 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) k_gather_histogram(co
     constexpr int P = KeyTraits<U>::kDigits;
     __shared__ __align__(16) uint32_t shall[gather_hist_copies<P>() * P * kBuckets];
     if constexpr (P >= 8) {
-        if (pa.prefix_ok)
-            prefix_sample_cta<U, THREADS>(reinterpret_cast<U *>(shall), n, ctrl, [&](uint64_t i) {
-                return filter_key<MODE>(gathered_key<U>(ptrs, i, off1, off2, level, keys_in));
-            });
+        if (pa.prefix_ok) {
+            gather_sample<U, MODE, THREADS>(reinterpret_cast<U *>(shall), ptrs, n, off1, off2, level, keys_in, ctrl);
+            __syncthreads();
+        }
     }
     zero_hist<THREADS, P>(shall);
     uint32_t *sh = shall + ((threadIdx.x >> 5) % gather_hist_copies<P>()) * P * kBuckets;

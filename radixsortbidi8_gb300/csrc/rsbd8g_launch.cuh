@@ -151,7 +151,7 @@ cudaError_t launch_histogram_t(const Resolved &r, uint64_t n, const void *in, co
     } else {
         constexpr int P = KeyTraits<U>::kDigits;
         constexpr size_t smem = size_t(hist_lane_copies<P>()) * P * kBuckets * 4;
-        static_assert(kHistDirectThreads * sizeof(U) <= smem, "the sample fits the counters' memory");
+        static_assert(kSampleDirect <= kHistDirectThreads && kSampleDirect * sizeof(U) <= smem, "the sample fits the counters' memory");
         auto kern = k_histogram<U, MODE, kHistDirectThreads>;
         histogram_setup<U, MODE>(dev);
         const uint64_t per = uint64_t(kHistDirectThreads) * 16;   // at least 16 keys a thread

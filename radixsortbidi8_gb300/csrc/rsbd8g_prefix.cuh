@@ -37,20 +37,31 @@ struct PlanArgs {
 // The settle step compares a key with its whole group, so its work grows with the group size: up to
 // this many equal-prefix keys on average are left to it.
 constexpr uint64_t kSettleGroup = 2;
-// the copies of one key that are walked over when the sample's pairs are counted
+// the copies of one key that count when the sample's pairs are weighted (a window of positions fits a word)
 constexpr uint32_t kSampleRun = 32;
 
-// Every CTA of the histogram launch sorts one key per thread, drawn at random places (independent
+// Every CTA of the histogram launch sorts up to a key per thread, drawn at random places (independent
 // draws, so an input that is already in order is judged as any other), and counts the pairs of
 // neighbours that differ, weighted with the copies each of the two has, by the highest digit in which
 // they differ.  Many small samples tell as much about equal prefixes as one large one of as many
 // pairs, and sort side by side: a bitonic network, by shuffles within a warp and through shared memory
-// beyond (one 8192-key sample on a CTA of its own took 70 us; these take 3).
-// The pairs that a sample can form should outnumber the keys, for one pair too many to show: a round of
-// samples for every 2^26 keys (152 samples of 1024 keys form 80 M pairs)
-__device__ __forceinline__ uint32_t prefix_rounds(uint64_t n) {
-    const uint64_t r = n >> 26;
-    return r < 1 ? 1u : r > 16 ? 16u : uint32_t(r);
+// beyond.
+// The pairs that the samples can form should outnumber the keys, for one pair too many to show: the smallest
+// size of sample that does (152 samples of 256 keys form 5 M pairs, of 1024 keys 80 M), or several rounds of the
+// largest.  A sample of 1024 keys adds 9 us to the histogram, of 256 keys 4 to 5 (2^21 int64 keys 28.4 -> 24.4 us, 19.1
+// without samples).
+constexpr int kSampleLeast = 256, kSampleDirect = 1024;    // k_histogram: up to one key per thread
+constexpr int kSampleGather = 512;                         // k_gather_histogram: one key per thread (smaller samples took as long)
+__host__ __device__ __forceinline__ uint64_t prefix_pairs(uint32_t samples, uint32_t size) { return uint64_t(samples) * (size * (size - 1u) / 2u); }
+template <int LEAST, int MOST>
+__host__ __device__ __forceinline__ uint32_t prefix_size(uint64_t n, uint32_t samples) {
+    uint32_t size = LEAST;
+    while (size < MOST && prefix_pairs(samples, size) < n) size *= 2;
+    return size;
+}
+__host__ __device__ __forceinline__ uint32_t prefix_rounds(uint64_t n, uint32_t samples, uint32_t size) {
+    const uint64_t r = n / prefix_pairs(samples, size) + 1u;
+    return r > 16 ? 16u : uint32_t(r);
 }
 template <typename U>
 __device__ __forceinline__ U shfl_key(U k, int mask) { return __shfl_xor_sync(0xFFFFFFFFu, k, mask); }
@@ -70,50 +81,90 @@ template <int HB>
 __device__ __forceinline__ KeyWide<HB> shfl_down_key(KeyWide<HB> k) {
     return KeyWide<HB>{__shfl_down_sync(0xFFFFFFFFu, k.lo, 1), __shfl_down_sync(0xFFFFFFFFu, k.hi, 1)};
 }
-template <typename U, int THREADS, typename F>
-__device__ __forceinline__ void prefix_sample(U *s, uint64_t n, uint32_t rounds, uint64_t first, uint32_t *pairs, F key) {
-    static_assert((THREADS & (THREADS - 1)) == 0, "a bitonic network of one key per thread");
-    const int i = threadIdx.x;
-    if (i < kMaxPasses) pairs[i] = 0;
+// the threads of a sample
+template <int SIZE, int THREADS>
+__device__ __forceinline__ void sample_sync() {
+    if constexpr (SIZE == THREADS) __syncthreads();
+    else asm volatile("bar.sync 2, %0;" ::"n"(SIZE) : "memory");
+}
+
+// where draw `index` lies among n keys (splitmix64 of its index)
+__device__ __forceinline__ uint64_t sample_place(uint64_t index, uint64_t n) {
+    uint64_t z = (index + 1u) * 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return __umul64hi(z ^ (z >> 31), n);
+}
+
+// `rounds` samples of SIZE keys, by the first SIZE threads of a CTA of THREADS; the round that enough() ends is
+// the last.  s: SIZE keys; heads: SIZE / 32 + 1 words; DRAWN: a0 is this thread's key of the first round
+template <int SIZE, int THREADS, bool DRAWN, typename U, typename F, typename E>
+__device__ __forceinline__ void prefix_sample(U *s, uint32_t *heads, uint64_t n, uint32_t rounds, uint64_t first, uint32_t *pairs, U a0,
+                                              F key, E enough) {
+    static_assert((SIZE & (SIZE - 1)) == 0, "a bitonic network of one key per thread");
+    constexpr uint32_t size = SIZE;
+    const uint32_t i = threadIdx.x;
+    if (i < uint32_t(kMaxPasses)) pairs[i] = 0;
+    if (i == 0) heads[size / 32] = 0xFFFFFFFFu;
     for (uint32_t round = 0; round < rounds; ++round) {
-        // splitmix64 of the sample's index
-        uint64_t z = ((first + round) * THREADS + i + 1u) * 0x9E3779B97F4A7C15ull;
-        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-        U a = key(__umul64hi(z ^ (z >> 31), n));
-        for (int k = 2; k <= THREADS; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
+        U a = DRAWN && round == 0 ? a0 : key(sample_place((first + round) * size + i, n));
+        for (uint32_t k = 2; k <= size; k <<= 1) {
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
                 U b;
                 if (j >= 32) {
-                    __syncthreads();
+                    sample_sync<SIZE, THREADS>();
                     s[i] = a;
-                    __syncthreads();
+                    sample_sync<SIZE, THREADS>();
                     b = s[i ^ j];
                 } else {
-                    b = shfl_key(a, j);
+                    b = shfl_key(a, int(j));
                 }
                 const bool low = ((i & j) == 0) == ((i & k) == 0);      // this thread keeps the smaller key
                 if (low ? key_less(b, a) : key_less(a, b)) a = b;
             }
         }
-        __syncthreads();
+        sample_sync<SIZE, THREADS>();
         s[i] = a;
-        __syncthreads();
-        if (i > 0 && !key_same(s[i - 1], a)) {
-            uint32_t before = 1, after = 1;
-            while (before < kSampleRun && i - 1 - int(before) >= 0 && key_same(s[i - 1 - int(before)], s[i - 1])) ++before;
-            while (after < kSampleRun && i + int(after) < THREADS && key_same(s[i + int(after)], a)) ++after;
-            atomicAdd(pairs + top_diff(s[i - 1], a), before * after);
+        sample_sync<SIZE, THREADS>();
+        const U prev = s[i ? i - 1 : 0];
+        const bool head = i == 0 || !key_same(prev, a);
+        const uint32_t hm = __ballot_sync(0xFFFFFFFFu, head);
+        if ((i & 31u) == 0) heads[i / 32] = hm;
+        sample_sync<SIZE, THREADS>();
+        if (head && i > 0) {
+            // the copies of the key before (the head at or before i - 1) and of this one (the next head), from the
+            // heads of the 32 positions on either side
+            const uint32_t w = i / 32, l = i & 31u;
+            const uint32_t below = uint32_t(((uint64_t(heads[w]) << 32) | (w ? heads[w - 1] : 0u)) >> l);
+            const uint32_t above = uint32_t(((uint64_t(heads[w + 1]) << 32) | heads[w]) >> (l + 1));
+            const uint32_t before = below ? uint32_t(__clz(below)) + 1u : kSampleRun, after = above ? uint32_t(__ffs(above)) : kSampleRun;
+            atomicAdd(pairs + top_diff(prev, a), before * after);
         }
-        __syncthreads();                                               // s is free again
+        sample_sync<SIZE, THREADS>();                                             // s and heads are free again
+        if (round + 1 < rounds && enough()) break;
     }
 }
-// the samples of one histogram CTA, added to the sort's
-template <typename U, int THREADS, typename F>
-__device__ __forceinline__ void prefix_sample_cta(U *s, uint64_t n, Control *__restrict__ ctrl, F key) {
-    __shared__ uint32_t pairs[kMaxPasses];
-    const uint32_t rounds = prefix_rounds(n);
-    prefix_sample<U, THREADS>(s, n, rounds, uint64_t(blockIdx.x) * rounds, pairs, key);
+// a thread's first key of the samples of its CTA (below)
+template <typename U, int LEAST, int MOST, typename F>
+__device__ __forceinline__ U prefix_draw(uint64_t n, F key) {
+    const uint32_t size = prefix_size<LEAST, MOST>(n, gridDim.x), rounds = prefix_rounds(n, gridDim.x, size);
+    return threadIdx.x < size ? key(sample_place(uint64_t(blockIdx.x) * rounds * size + threadIdx.x, n)) : U{};
+}
+// the samples of one histogram CTA, of LEAST to MOST keys, added to the sort's; a0: the thread's first key (if the size
+// is not a fixed one)
+template <typename U, int THREADS, int LEAST, int MOST, typename F>
+__device__ __forceinline__ void prefix_sample_cta(U *s, uint64_t n, Control *__restrict__ ctrl, U a0, F key) {
+    __shared__ uint32_t pairs[kMaxPasses], heads[MOST / 32 + 1];
+    const uint32_t size = prefix_size<LEAST, MOST>(n, gridDim.x), rounds = prefix_rounds(n, gridDim.x, size);
+    const uint64_t first = uint64_t(blockIdx.x) * rounds;
+    auto all = [] { return false; };
+    if (threadIdx.x < size) {
+        if (LEAST == MOST || size == MOST) prefix_sample<MOST, THREADS, LEAST != MOST>(s, heads, n, rounds, first, pairs, a0, key, all);
+        else if (size == LEAST) prefix_sample<LEAST, THREADS, true>(s, heads, n, rounds, first, pairs, a0, key, all);
+        else prefix_sample<2 * LEAST, THREADS, true>(s, heads, n, rounds, first, pairs, a0, key, all);
+    }
+    static_assert(LEAST == MOST || MOST == 4 * LEAST, "the sizes between");
+    __syncthreads();
     if (threadIdx.x < kMaxPasses && pairs[threadIdx.x]) atomicAdd(&ctrl->sample_pairs[threadIdx.x], pairs[threadIdx.x]);
 }
 
@@ -137,6 +188,14 @@ __device__ __forceinline__ uint32_t prefix_choose(const uint32_t *sample_pairs, 
         pairs += sample_pairs[q];
     }
     return k;
+}
+// will prefix_choose find none, whatever pairs are still to come?
+__device__ __forceinline__ bool prefix_hopeless(const uint32_t *sample_pairs, uint32_t survive, uint64_t n, uint64_t all) {
+    const int most = min(__popc(survive) - 2, kPrefixSlots);
+    uint64_t pairs = 0;
+    int q = 0;
+    for (; q < kMaxPasses && !(((survive >> q) & 1u) && __popc(survive >> q) <= most); ++q) pairs += sample_pairs[q];
+    return (pairs + 1u) * n > kSettleGroup * all;
 }
 
 // Plan the passes over the digits of `mask`, lowest first, from array `cur` on; returns where they
