@@ -20,18 +20,21 @@ struct Resolved {
     uint32_t digits;      // 8-bit digit passes of the key
     uint32_t elem_bytes;  // bytes per array element (key bytes, or 8 for object pointers)
     uint32_t indirect;    // RSBD8G_DIRECT / RSBD8G_MEMBER / RSBD8G_MEMBER2
-    uint32_t flags;
+    uint32_t flags;       // RSBD8G_FLAG_* of the descriptor (other bits of it mean nothing)
+    uint32_t shared_gpu;  // a served batch: its kernels share the GPU with other streams'
     uint32_t prefetch;    // every array of the call is device memory (tiles may be prefetched into L2)
     int64_t off1, off2;
     const void *keys;     // RSBD8G_KEYED: the caller's key array
 };
 
-// Resolved::flags of a batch whose kernels share the GPU with other streams' (the server sets it): it is not
-// sorted by a prefix, as the launches that leaves idle would each wait for their CTAs' turn behind
-// another stream's passes (29 mixed requests of up to 2^22 keys: 1.22-1.29 ms with them, 1.11 without; one
-// large request alone still gains more than it waits: 48 requests of up to 2^24 keys 2.85 ms, 3.07 without).
-// The same bit is named in rsbd8g_serve.cpp.
-constexpr uint32_t kFlagSharedGpu = 1u << 30;
+// A batch whose kernels share the GPU with other streams' (Resolved::shared_gpu) is not sorted by a prefix, as the
+// launches that leaves idle would each wait for their CTAs' turn behind another stream's passes (29 mixed
+// requests of up to 2^22 keys: 1.22-1.29 ms with them, 1.11 without; one large request alone still gains
+// more than it waits: 48 requests of up to 2^24 keys 2.85 ms, 3.07 without).  The server's batches come in here:
+rsbd8g_status segmented_shared_gpu(const rsbd8g_desc *desc, size_t total, size_t nsegs, const uint64_t *offsets,
+                                   const uint64_t *input_ptrs, const uint64_t *output_ptrs, const uint64_t *buffer_ptrs,
+                                   const uint8_t *directions, void *scratch, size_t scratch_bytes,
+                                   const rsbd8g_segtuning *tuning, rsbd8g_stream stream);
 
 // byte offsets of the parts of a scratch area
 struct Layout {

@@ -148,7 +148,7 @@ template <typename U, int MODE>
 cudaError_t launch_segmented_mode_t(const Resolved &r, const SegArgs &args, const SegLayout &L, unsigned char *scratch,
                                     const void *in_, void *out_, void *buf_, cudaStream_t s) {
     SegArgs a = args;
-    a.prefix_ok = KeyTraits<U>::kDigits >= 8 && a.total >= prefix_min_keys(int(sizeof(U))) && !(r.flags & (RSBD8G_FLAG_DIAG_STALL | kFlagSharedGpu));
+    a.prefix_ok = KeyTraits<U>::kDigits >= 8 && a.total >= prefix_min_keys(int(sizeof(U))) && !(r.flags & RSBD8G_FLAG_DIAG_STALL) && !r.shared_gpu;
     const U *in = static_cast<const U *>(in_);
     U *out = static_cast<U *>(out_);
     U *buf = static_cast<U *>(buf_);

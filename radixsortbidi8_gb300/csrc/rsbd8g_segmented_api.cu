@@ -80,10 +80,11 @@ static rsbd8g_status segmented_common(const rsbd8g_desc *desc, size_t total, siz
                                       void *scratch, size_t scratch_bytes, const void *input, void *output,
                                       void *buffer, const uint64_t *in_ptrs, const uint64_t *out_ptrs,
                                       const uint64_t *buf_ptrs, const uint8_t *seg_dirs, const rsbd8g_segtuning *tuning,
-                                      rsbd8g_stream stream) {
+                                      rsbd8g_stream stream, bool shared_gpu = false) {
     Resolved r;
     rsbd8g_status st = resolve(desc, &r);
     if (st != RSBD8G_OK) return st;
+    r.shared_gpu = shared_gpu;
     if (r.indirect != RSBD8G_DIRECT || r.x87) return RSBD8G_ERR_BAD_ARG;
     if (nsegs == 0 || total == 0) return RSBD8G_OK;
     if (!offsets || !scratch) return RSBD8G_ERR_BAD_ARG;
@@ -178,3 +179,12 @@ RSBD8G_API rsbd8g_status rsbd8g_segmented_sortcopy_ptrs_dirs(const rsbd8g_desc *
 }
 
 }  // extern "C"
+
+rsbd8g_status rsbd8g::segmented_shared_gpu(const rsbd8g_desc *desc, size_t total, size_t nsegs, const uint64_t *offsets,
+                                           const uint64_t *input_ptrs, const uint64_t *output_ptrs,
+                                           const uint64_t *buffer_ptrs, const uint8_t *directions, void *scratch,
+                                           size_t scratch_bytes, const rsbd8g_segtuning *tuning, rsbd8g_stream stream) {
+    if (!directions && nsegs && total) return RSBD8G_ERR_BAD_ARG;
+    return segmented_common(desc, total, nsegs, offsets, scratch, scratch_bytes, nullptr, nullptr, nullptr,
+                            input_ptrs, output_ptrs, buffer_ptrs, directions, tuning, stream, true);
+}

@@ -31,12 +31,15 @@
 namespace rsbd8g {
 bool device_memory(const void *p);            // rsbd8g_api.cu
 int filter_class(const rsbd8g_desc *d);       // rsbd8g_api.cu
+rsbd8g_status segmented_shared_gpu(const rsbd8g_desc *desc, size_t total, size_t nsegs, const uint64_t *offsets,
+                                   const uint64_t *input_ptrs, const uint64_t *output_ptrs, const uint64_t *buffer_ptrs,
+                                   const uint8_t *directions, void *scratch, size_t scratch_bytes,
+                                   const rsbd8g_segtuning *tuning, rsbd8g_stream stream);     // rsbd8g_segmented_api.cu
 }
 
 namespace {
 
 constexpr size_t kAlignArena = 256;
-constexpr uint32_t kFlagSharedGpu = 1u << 30;     // rsbd8g_internal.h
 size_t aup(size_t x) { return (x + kAlignArena - 1) & ~(kAlignArena - 1); }
 
 // first-fit allocator over [0, size) of the arena; host bookkeeping only
@@ -336,7 +339,6 @@ struct Server {
         bool device = true;
         for (size_t i = 0; i < n; ++i) device = device && b->reqs[i]->device;
         if (device) key.flags |= RSBD8G_FLAG_DEVICE_ARRAYS;
-        key.flags |= kFlagSharedGpu;       // (batches overlap on the device)
         for (size_t i = 0; i < n; ++i) {
             ho[i + 1] = ho[i] + b->reqs[i]->count;
             hi[i] = reinterpret_cast<uint64_t>(b->reqs[i]->in);
@@ -364,9 +366,9 @@ struct Server {
             st = RSBD8G_ERR_CUDA;
         }
         else
-            st = rsbd8g_segmented_sortcopy_ptrs_dirs(&key, b->keys, n, d_off, d_in, d_out, d_buf, d_dir,
-                                                     arena_base + b->scratch_off, b->scratch_bytes, &tun,
-                                                     reinterpret_cast<rsbd8g_stream>(s));
+            st = rsbd8g::segmented_shared_gpu(&key, b->keys, n, d_off, d_in, d_out, d_buf, d_dir,      // (batches overlap
+                                              arena_base + b->scratch_off, b->scratch_bytes, &tun,     // on the device)
+                                              reinterpret_cast<rsbd8g_stream>(s));
         if (st == RSBD8G_OK &&
             cudaMemcpyAsync(b->host_err, arena_base + b->scratch_off, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess)
             st = RSBD8G_ERR_CUDA;

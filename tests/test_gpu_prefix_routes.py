@@ -259,3 +259,19 @@ def test_a_crowd_in_a_batch(kt, mode, direction, size, failed):
         assert same_bits(got[b:e], O.sortcopy(a[b:e].view(kt), mode, direction))
     first, second = seg_passes(s)
     assert first and not first & 1 and (second != 0) == bool(failed), (first, second)
+
+
+def test_unnamed_flag_bits_change_no_route():
+    """bits of the descriptor's flags that the header does not name are without meaning"""
+    import torch
+    from radixsortbidi8_gb300 import batched
+    n = 1 << 21
+    x = torch.from_numpy(S.uniform_bits(3, n, np.int64)).cuda()
+    offs = torch.tensor([0, n // 2, n], dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    seen = []
+    for flags in [0] + [1 << b for b in (4, 17, 30, 31)]:
+        s = batched.SegmentedSorter(x, offs, "ascfwdorder", "native", key_dtype=np.int64)
+        batched.segmented_sortcopy(x, s.output, s.buffer, offs, s.scratch, "ascfwdorder", "native", np.int64, s.tuning, s.stream, flags)
+        seen.append(seg_passes(s))
+    assert seen[0][0] and not seen[0][0] & 1 and all(p == seen[0] for p in seen), seen     # (a prefix, without the lowest digit)
