@@ -282,7 +282,7 @@ __device__ __forceinline__ void plan_copy(Control *__restrict__ ctrl, const Plan
 //   A group from an earlier chunk is otherwise left alone, as that chunk's warp settles it.  No inversion is passed
 // over: each lies in some warp's chunk, and its group either ends within the view of the chunk it starts in
 // or is taken by settle_long, which raises settle_fail where the group is too long.  Neighbouring chunks read keys
-// that a chunk moves only for their prefixes, which a move within a group leaves as they are.
+// that a chunk moves only for their prefixes, which a move within a group leaves as they are (settle_ld).
 template <typename U>
 struct SettleShape {
     static constexpr int kThreads = sizeof(U) == 8 ? 256 : 128;     // (static shared memory stays below 48 KB)
@@ -347,10 +347,44 @@ __device__ __forceinline__ int bit_at_or_above(const uint32_t *w, int i, int wor
     return m ? x * 32 + __ffs(m) - 1 : words * 32;
 }
 
-// ITEMS keys from p on: 16-byte loads where the address allows
-template <int ITEMS, typename U>
-__device__ __forceinline__ void load_run(U (&v)[ITEMS], const U *p) {
-    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+// the key as the sort orders it
+template <int MODE, typename U>
+__device__ __forceinline__ U settle_order(U b, bool desc) {
+    const U q = filter_key<MODE>(b);
+    return desc ? key_not(q) : q;
+}
+
+// Keys that another warp may be moving are read, and written, in one piece.  An 8-byte key is one access; of a 16-byte
+// key PTX promises that only for the 128-bit type.  Two words of different keys of a group do no harm where the order
+// is taken word by word: the group's prefix is in each.  Where a word's bits depend on the other's (a negation, a
+// shift: the float, absolute signed and tiered orders) they could show a prefix that no key has.
+template <int MODE, typename U>
+constexpr bool kWholeKeys = sizeof(U) == 16 && (MODE == 1 || MODE == 3 || MODE == 5 || MODE == 6);
+template <int MODE, typename U>
+__device__ __forceinline__ U settle_ld(const U *p) {
+    if constexpr (kWholeKeys<MODE, U>) {
+        U k;
+        asm volatile("{ .reg .b128 v; ld.relaxed.gpu.global.b128 v, [%2]; mov.b128 {%0, %1}, v; }" : "=l"(k.lo), "=l"(k.hi) : "l"(p) : "memory");
+        return k;
+    } else {
+        return *p;
+    }
+}
+template <int MODE, typename U>
+__device__ __forceinline__ void settle_st(U *p, U k) {
+    if constexpr (kWholeKeys<MODE, U>)
+        asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p), "l"(k.lo), "l"(k.hi) : "memory");
+    else
+        *p = k;
+}
+
+// ITEMS keys from p on: 16-byte loads where the address allows; whole: settle_ld
+template <int MODE, int ITEMS, typename U>
+__device__ __forceinline__ void load_run(U (&v)[ITEMS], const U *p, bool whole) {
+    if (kWholeKeys<MODE, U> && whole) {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) v[i] = settle_ld<MODE>(p + i);
+    } else if (sizeof(U) == 8 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
         constexpr int V = 16 / int(sizeof(U));
 #pragma unroll
         for (int i = 0; i < ITEMS; i += V) {
@@ -363,12 +397,6 @@ __device__ __forceinline__ void load_run(U (&v)[ITEMS], const U *p) {
     }
 }
 
-// the key as the sort orders it
-template <int MODE, typename U>
-__device__ __forceinline__ U settle_order(U b, bool desc) {
-    const U q = filter_key<MODE>(b);
-    return desc ? key_not(q) : q;
-}
 
 // take up the long group `id`: 1, or 0 if another warp has, -1 if the table is full
 template <typename U>
@@ -439,8 +467,8 @@ __device__ __noinline__ void settle_long(U *keys, uint64_t *vals, uint64_t at, u
     static_assert(sizeof(warp->key) >= 2 * kBuckets * 4, "the offsets and the next counts fit the view's memory");
     const int lane = int(threadIdx.x & 31u);
     const uint32_t limit = uint32_t(w.limit);
-    const U ref = settle_order<MODE>(keys[at], desc);
-    auto same = [&](uint64_t i) { return same_masked(settle_order<MODE>(keys[i], desc), ref, mask); };
+    const U ref = settle_order<MODE>(settle_ld<MODE>(keys + at), desc);
+    auto same = [&](uint64_t i) { return same_masked(settle_order<MODE>(settle_ld<MODE>(keys + i), desc), ref, mask); };
     const uint32_t back = warp_last(1, uint32_t(at < limit ? at : limit), [&](uint32_t d) { return same(at - d); });
     const uint32_t on = warp_last(0, uint32_t(n - 1 - at < limit ? n - 1 - at : limit), [&](uint32_t d) { return same(at + d); });
     const uint32_t len = back + on + 1;
@@ -520,7 +548,7 @@ __device__ __noinline__ void settle_long(U *keys, uint64_t *vals, uint64_t at, u
                 if (in && before == 0) off[d] += uint32_t(__popc(peers));
                 __syncwarp();
                 if (to < len) {
-                    dst[to] = k[q];
+                    settle_st<MODE>(dst + to, k[q]);
                     if constexpr (HAS_VAL) dst_v[to] = v[q];
                 }
                 if (in && next >= 0) atomicAdd(cnt + digit_of(b, next), 1u);
@@ -537,7 +565,7 @@ __device__ __noinline__ void settle_long(U *keys, uint64_t *vals, uint64_t at, u
     if (src != keys + s) {
 #pragma unroll 4
         for (uint32_t x = uint32_t(lane); x < len; x += 32) {
-            dst[x] = src[x];
+            settle_st<MODE>(dst + x, src[x]);
             if constexpr (HAS_VAL) dst_v[x] = src_v[x];
         }
     }
@@ -553,13 +581,13 @@ __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, u
     uint32_t *hw = warp->head, *vw = warp->inv;
     const int lane = int(threadIdx.x & 31u);
     const int view = int(n - c0 < uint64_t(S::kView) ? n - c0 : uint64_t(S::kView));
-    for (int x = lane; x < view; x += 32) key[x] = keys[c0 + x];
+    for (int x = lane; x < view; x += 32) key[x] = settle_ld<MODE>(keys + c0 + x);
     __syncwarp();
     for (int w = 0; w < WORDS; ++w) {
         const int x = w * 32 + lane;
         bool h = x == 0 ? c0 == 0 : x >= view, v = false;
         if (!h) {
-            const U a = settle_order<MODE>(x ? key[x ? x - 1 : 0] : keys[c0 - 1], desc), b = settle_order<MODE>(key[x], desc);
+            const U a = settle_order<MODE>(x ? key[x ? x - 1 : 0] : settle_ld<MODE>(keys + c0 - 1), desc), b = settle_order<MODE>(key[x], desc);
             h = !same_masked(a, b, mask);
             v = !h && key_less(b, a);
         }
@@ -596,7 +624,7 @@ __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, u
                 const U a = settle_order<MODE>(key[j], desc);
                 at += key_less(a, b) || (j < i && key_same(a, b)) ? 1 : 0;
             }
-            keys[c0 + at] = key[i];
+            settle_st<MODE>(keys + c0 + at, key[i]);
             if constexpr (HAS_VAL) vals[c0 + at] = p[r];
         }
         s = e;
@@ -618,39 +646,46 @@ __device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c
     const bool full = n - c0 >= uint64_t(32 * ITEMS);
     const int own = full ? ITEMS : int(n - c0) - lane * ITEMS;      // this lane's keys (may be < 0 or > ITEMS)
     U v[ITEMS], before{};
-    if (full) {
-        load_run<ITEMS>(v, keys + c0 + lane * ITEMS);
-    } else {
+    uint32_t hb, vb, heads;
+    for (bool whole = false;; whole = true) {
+        if (full) {
+            load_run<MODE, ITEMS>(v, keys + c0 + lane * ITEMS, whole || lane == 0 || lane == 31);
+        } else {
 #pragma unroll
-        for (int j = 0; j < ITEMS; ++j) {
-            v[j] = U{};
-            if (j < own) v[j] = keys[c0 + lane * ITEMS + j];
+            for (int j = 0; j < ITEMS; ++j) {
+                v[j] = U{};
+                if (j < own) v[j] = settle_ld<MODE>(keys + c0 + lane * ITEMS + j);
+            }
         }
-    }
-    if (lane == 0 && c0) before = keys[c0 - 1];
-    if constexpr (!RAW) {
-        before = settle_order<MODE>(before, desc);
+        before = lane == 0 && c0 ? settle_ld<MODE>(keys + c0 - 1) : U{};
+        if constexpr (!RAW) {
+            before = settle_order<MODE>(before, desc);
 #pragma unroll
-        for (int j = 0; j < ITEMS; ++j) v[j] = settle_order<MODE>(v[j], desc);
-    }
-    // heads and inversions among this lane's keys (bit j: key j)
-    uint32_t hb = 0, vb = 0;
-    {
-        const U up = shfl_up_key(v[ITEMS - 1]);
-        U a = ordered(lane ? up : before);
-#pragma unroll
-        for (int j = 0; j < ITEMS; ++j) {
-            const U b = ordered(v[j]);
-            const bool h = !same_masked(a, b, mask);
-            if (h) hb |= 1u << j;
-            else if (key_less(b, a)) vb |= 1u << j;
-            a = b;
+            for (int j = 0; j < ITEMS; ++j) v[j] = settle_order<MODE>(v[j], desc);
         }
+        // heads and inversions among this lane's keys (bit j: key j)
+        hb = vb = 0;
+        {
+            const U up = shfl_up_key(v[ITEMS - 1]);
+            U a = ordered(lane ? up : before);
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) {
+                const U b = ordered(v[j]);
+                const bool h = !same_masked(a, b, mask);
+                if (h) hb |= 1u << j;
+                else if (key_less(b, a)) vb |= 1u << j;
+                a = b;
+            }
+        }
+        if (c0 == 0 && lane == 0) hb |= 1u;
+        if (!full) hb |= own >= ITEMS ? 0u : own <= 0 ? 0xFFu : 0xFFu << own;     // past the end: each alone
+        vb &= ~hb;
+        heads = __ballot_sync(0xFFFFFFFFu, hb != 0);
+        // Another warp moves keys here only of a group that came in or of one that runs far past the halo.  The first and
+        // the last lane's keys, which are read whole, tell: a head in the first, and one after the last's first key.
+        if (!kWholeKeys<MODE, U> || !full || whole) break;
+        if ((heads & 1u) && __any_sync(0xFFFFFFFFu, lane == 31 && (hb & 0xFEu))) break;
     }
-    if (c0 == 0 && lane == 0) hb |= 1u;
-    if (!full) hb |= own >= ITEMS ? 0u : own <= 0 ? 0xFFu : 0xFFu << own;     // past the end: each alone
-    vb &= ~hb;
-    const uint32_t heads = __ballot_sync(0xFFFFFFFFu, hb != 0);
     const bool open = !(heads >> 31) && (heads & 0x7FFFFFFFu) && n - c0 > uint64_t(32 * ITEMS);
     if (!__any_sync(0xFFFFFFFFu, vb != 0) && !open) return;
     // this lane's keys of the group that came in, and of the groups that the next chunk settles
@@ -662,7 +697,7 @@ __device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c
         // met by the chunk before too, if it holds the start and has the inversion in its view
         bool left = bad_in && lane * ITEMS + 31 - __clz(bad_in) >= S::kView - C;
         if (bad_in && c0 > uint64_t(C)) {
-            const U a = settle_order<MODE>(keys[c0 - C - 1], desc), b = settle_order<MODE>(keys[c0 - 1], desc);
+            const U a = settle_order<MODE>(settle_ld<MODE>(keys + c0 - C - 1), desc), b = settle_order<MODE>(settle_ld<MODE>(keys + c0 - 1), desc);
             left |= same_masked(a, b, mask);
         }
         if (left) settle_later(warp, c0 + uint64_t(lane * ITEMS + 31 - __clz(bad_in)), fail, fail_bit);
@@ -742,7 +777,7 @@ __device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c
             }
 #pragma unroll
             for (int j = 0; j < ITEMS; ++j)
-                if ((moved >> j) & 1u) dst[j] = v[j];
+                if ((moved >> j) & 1u) settle_st<MODE>(dst + j, v[j]);
         }
     }
     if (wide) settle_wide<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc, warp, fail, fail_bit);

@@ -218,9 +218,12 @@ def test_a_crowd_of_pointers(size, failed, direction):
 
 
 @pytest.mark.parametrize("size,failed", [(1500, 0), (2000, 0), (30000, 1)])
-@pytest.mark.parametrize("kind,mode,direction", [("u128", "native", "dscfwdorder"), ("f128", "native", "ascrevorder"), ("x87", "nativeabs", "ascrevorder")])
+@pytest.mark.parametrize("kind,mode,direction", [("u128", "native", "dscfwdorder"), ("f128", "native", "ascrevorder"), ("x87", "nativeabs", "ascrevorder"),
+                                                 ("u128", 3, "dscrevorder"), ("u128", 1, "ascfwdorder"), ("f128", 5, "dscfwdorder"),
+                                                 ("x87", "native", "dscrevorder")])
 def test_a_crowd_of_16_byte_keys(size, failed, kind, mode, direction):
-    """(settle_limit is 2048 of 2^20 keys)"""
+    """(settle_limit is 2048 of 2^20 keys; modes 3, 1, 5 and the float order carry from word to word: half of the keys
+    of the absolute signed mode are negated, some with a low word of zero)"""
     import torch
     import radixsortbidi8_gb300 as rs
     n = 1 << 20
@@ -232,6 +235,10 @@ def test_a_crowd_of_16_byte_keys(size, failed, kind, mode, direction):
     else:
         w = np.stack([lo, hi], axis=1)
     w[at] = w[at[np.arange(at.size) // 2 * 2]]            # ties
+    if mode == 3:
+        w[at[::8], 0] = 0
+        w[1::2, 1] = ~w[1::2, 1] + (w[1::2, 0] == 0)
+        w[1::2, 0] = ~w[1::2, 0] + np.uint64(1)
     x = torch.from_numpy(w.view(np.int64).reshape(-1)).cuda()
     y, buf = torch.empty_like(x), torch.empty_like(x)
     scratch = torch.empty(rs.scratch_bytes(kind, n, direction, mode), dtype=torch.uint8, device="cuda")
