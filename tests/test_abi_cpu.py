@@ -140,8 +140,9 @@ def test_plan_numbers_from_scratch_are_in_range(tmp_path):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("no nvcc")
+    from radixsortbidi8_gb300 import build as B
     exe = str(tmp_path / "plan_range_test")
-    r = subprocess.run([nvcc, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "radixsortbidi8_gb300", "csrc"),
+    r = subprocess.run([nvcc, *B.ARCH, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "radixsortbidi8_gb300", "csrc"),
                         os.path.join(ROOT, "tests", "cpp", "plan_range_test.cu"), "-o", exe], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     r = subprocess.run([exe], capture_output=True, text=True)
