@@ -98,6 +98,9 @@ enum {
  * pointer-table form prefetches only with this flag.  Managed and host memory are read with plain
  * loads alone. */
 #define RSBD8G_FLAG_DEVICE_ARRAYS 4u
+/* diagnostics only: the sort runs as a launch per digit, never as one kernel (the route that a small
+ * sort takes where a cooperative launch does not fit) */
+#define RSBD8G_FLAG_DIAG_LAUNCHES 8u
 
 typedef struct rsbd8g_desc {
     uint32_t key_bytes;     /* 1, 2, 4, 8 or 16 (x87 keys: not in the segmented and serving entry points) */

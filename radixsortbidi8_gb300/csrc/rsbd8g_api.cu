@@ -162,7 +162,7 @@ rsbd8g_status resolve(const rsbd8g_desc *d, Resolved *r) {
     r->elem_bytes = d->indirection ? 8u : d->key_bytes;
     r->off1 = d->offset1;
     r->off2 = d->offset2;
-    r->flags = d->flags & (RSBD8G_FLAG_DIAG_STALL | RSBD8G_FLAG_DIAG_NOMEM | RSBD8G_FLAG_DEVICE_ARRAYS);
+    r->flags = d->flags & (RSBD8G_FLAG_DIAG_STALL | RSBD8G_FLAG_DIAG_NOMEM | RSBD8G_FLAG_DEVICE_ARRAYS | RSBD8G_FLAG_DIAG_LAUNCHES);
     r->shared_gpu = 0;
     r->prefetch = 0;
     r->keys = nullptr;

@@ -121,7 +121,7 @@ bool launch_one_mode(const OneCall &c, cudaError_t *e) {
 template <typename U>
 bool launch_one_t(const Resolved &r, uint64_t n, unsigned char *scratch, size_t scratch_bytes, const void *in, void *out,
                   void *buf, const Layout &L, bool inplace, bool to_buffer, cudaStream_t s, cudaError_t *e) {
-    if (n >= kOneMaxKeys || (r.flags & RSBD8G_FLAG_DIAG_STALL)) return false;
+    if (n >= kOneMaxKeys || (r.flags & (RSBD8G_FLAG_DIAG_STALL | RSBD8G_FLAG_DIAG_LAUNCHES))) return false;
     OneCall c{};
     c.n = n;
     c.scratch = scratch;

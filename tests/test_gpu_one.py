@@ -105,3 +105,34 @@ def test_captured_in_a_graph(n):
         g.replay()
     s.synchronize()
     assert same_bits(from_dev(y, np.uint32), O.sortcopy(a))
+
+
+@pytest.mark.parametrize("n", [2, 31, 2047, 4096, 4097, 8192, 8193, 100003, 300007])
+@pytest.mark.parametrize("dtype,mode,direction", [(np.uint8, "native", "ascfwdorder"), (np.int16, "nativetieredabs", "dscfwdorder"),
+                                                  (np.uint32, "native", "dscfwdorder"), (np.float32, "nativeabs", "dscrevorder"),
+                                                  (np.int64, "native", "ascfwdorder"), (np.float64, "native", "ascrevorder")],
+                         ids=lambda x: str(getattr(x, "__name__", x)))
+def test_small_sorts_by_a_launch_per_digit(dtype, mode, direction, n):
+    """the route of small sorts where no cooperative launch fits, and that it is the one taken"""
+    import torch
+    import radixsortbidi8_gb300 as rs
+    from radixsortbidi8_gb300 import api
+    a = keys(dtype, n, n)
+    want = O.sortcopy(a, mode, direction)
+    x, y = to_dev(a), empty_dev(n, dtype)
+    api.profile_enable(True)
+    assert rs.radixsortcopy(x, y, direction, mode, key_dtype=dtype, flags=api.FLAG_DIAG_LAUNCHES)
+    api.profile_enable(False)
+    ran = [r["kernel"] for r in api.profile_collect()]
+    assert "histogram" in ran and ran.count("onesweep") == np.dtype(dtype).itemsize and "one" not in ran, ran
+    assert same_bits(from_dev(y, dtype), want)
+    assert rs.radixsort(x, direction, mode, key_dtype=dtype, flags=api.FLAG_DIAG_LAUNCHES)
+    assert same_bits(from_dev(x, dtype), want)
+    key = keys(dtype, n, n + 1)
+    rec = np.zeros((n, 24 // key.itemsize), dtype=dtype)
+    rec[:, 8 // key.itemsize] = key
+    dev = torch.from_numpy(rec.view(np.int64)).cuda()
+    ptr = dev.data_ptr() + 24 * torch.arange(n, dtype=torch.int64, device="cuda")
+    out = torch.empty_like(ptr)
+    assert rs.radixsortcopy_member(ptr, out, dtype, 8, direction, mode, flags=api.FLAG_DIAG_LAUNCHES)
+    assert np.array_equal((out.cpu().numpy() - dev.data_ptr()) // 24, O.numpy_sort_indices(key, mode, direction))

@@ -282,3 +282,64 @@ def test_unnamed_flag_bits_change_no_route():
         batched.segmented_sortcopy(x, s.output, s.buffer, offs, s.scratch, "ascfwdorder", "native", np.int64, s.tuning, s.stream, flags)
         seen.append(seg_passes(s))
     assert seen[0][0] and not seen[0][0] & 1 and all(p == seen[0] for p in seen), seen     # (a prefix, without the lowest digit)
+
+
+@pytest.mark.parametrize("kt,mode", [(np.int64, "native"), (np.float64, "nativeabs")], ids=str)
+def test_pointer_tables_and_directions_with_a_prefix(kt, mode):
+    """batches of separate arrays, each with its direction: settled segments, a crowd in the view's length and one
+    too long, reversed ties, small segments beside them"""
+    import torch
+    from radixsortbidi8_gb300 import batched
+    arrs = [segment(600011, 1500, 0, 3), S.uniform_bits(5, 700001, np.uint64), segment(600011, 30000, 2, 7), S.uniform_bits(6, 5000, np.uint64),
+            S.uniform_bits(8, 250007, np.uint64), segment(300011, 700, 5, 9)]
+    arrs = [(a & np.uint64((1 << 63) - 1)).view(np.int64) for a in arrs]
+    for a in arrs:
+        at = np.flatnonzero(a >> 24 == 0x77777777)
+        a[at] = a[at[np.arange(at.size) // 4 * 4]]
+        if mode == "nativeabs":
+            a[1::2] |= np.int64(-1 << 63)
+    dirs = ["ascfwdorder", "dscrevorder", "dscfwdorder", "ascrevorder", "ascrevorder", "dscrevorder"]
+    ins = [torch.from_numpy(a).cuda() for a in arrs]
+    outs, bufs = [torch.empty_like(x) for x in ins], [torch.empty_like(x) for x in ins]
+    total = sum(a.size for a in arrs)
+    assert total >= 1 << 21                                # (a prefix is possible)
+    scratch = torch.empty(batched.segmented_scratch_bytes(kt, total, len(arrs), "ascfwdorder", mode), dtype=torch.uint8, device="cuda")
+    keep = batched.segmented_sortcopy_ptrs(ins, outs, bufs, scratch, mode=mode, key_dtype=kt, directions=dirs)
+    torch.cuda.synchronize()
+    first, second = [int(v) for v in scratch[152:160].cpu().numpy().view(np.uint32)]
+    assert first and not first & 1 and second, (first, second)
+    for a, d, y in zip(arrs, dirs, outs):
+        assert same_bits(y.cpu().numpy().view(kt), O.sortcopy(a.view(kt), mode, d))
+    del keep
+
+
+def places(n, draws):
+    """sampled() of many draws of fewer than 2^32 keys"""
+    z = (np.arange(1, draws + 1, dtype=np.uint64)) * np.uint64(0x9E3779B97F4A7C15)
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    z ^= z >> np.uint64(31)
+    low = np.uint64(0xFFFFFFFF)
+    return (((z >> np.uint64(32)) * np.uint64(n) + ((z & low) * np.uint64(n) >> np.uint64(32))) >> np.uint64(32)).astype(np.int64)
+
+
+@pytest.mark.parametrize("size,failed", [(60000, 0), (300000, 1)])
+def test_a_crowd_with_wide_look_back_words(size, failed):
+    """2^30 keys and more: 8-byte look-back words, settle_limit 131,072; the order is torch.sort's"""
+    import torch
+    import radixsortbidi8_gb300 as rs
+    n = (1 << 30) + 5
+    assert np.array_equal(places(1000003, 500), sampled(1000003, 500))
+    at = np.arange(size, dtype=np.int64) * 3001 + 11
+    at = at[~np.isin(at, places(n, 160 * 1024 * 16))]     # 16 rounds at most
+    assert at.size > size * 0.9
+    x = S.uniform_bits_torch(3, n, 8)
+    p = torch.from_numpy(at).cuda()
+    x[p] = (x[p] & 0xFFFFFF) | 0x0077777777000000
+    y, buf = torch.empty_like(x), torch.empty_like(x)
+    scratch = torch.empty(rs.scratch_bytes(np.int64, n), dtype=torch.uint8, device="cuda")
+    rs.radixsortcopynoalloc(x, y, buf, scratch, key_dtype=np.int64)
+    q = plan_of(scratch)
+    assert q["passes"] > 0 and q["failed"] == failed and q["error"] == 0, q
+    del buf, scratch
+    assert torch.equal(y, torch.sort(x)[0])
