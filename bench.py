@@ -157,10 +157,22 @@ def make_arrays(log2n: int, device):
     return S.sweep_arrays_torch(1 << log2n, device=device)
 
 
-def passes_that_ran(sweep_ms) -> list:
-    """The times of the scatter launches that moved keys: a pass that the plan skips returns at once."""
-    top = max((ms for _, ms in sweep_ms), default=0.0)
-    return [ms for _, ms in sweep_ms if ms > top / 8]
+# the control block at the start of a plain sort's scratch (Control, PassPlan of rsbd8g_device.cuh), in 32-bit words
+CTRL_PLAN, PLAN_WORDS, PLAN_ACTIVE, CTRL_SLOTS = 72, 8, 4, 22
+
+
+def planned_slots(scratch) -> set:
+    """The scatter launches of the last sort with this scratch whose plan had them move keys."""
+    import numpy as np
+    w = scratch[:4 * (CTRL_PLAN + PLAN_WORDS * CTRL_SLOTS)].cpu().numpy().view(np.uint32)[CTRL_PLAN:]
+    return {i for i in range(CTRL_SLOTS) if w[PLAN_WORDS * i + PLAN_ACTIVE]}
+
+
+def passes_that_ran(sweep_ms, slots, steps: int) -> list:
+    """The times of the scatter launches that moved keys, of (launch slot, ms) records of `steps` sorts."""
+    ran = [ms for p, ms in sweep_ms if p in slots]
+    assert len(ran) == steps * len({p for p, _ in sweep_ms} & slots), "a launch per step and slot"
+    return ran
 
 
 def active_passes(bits, name: str) -> int:
@@ -249,6 +261,7 @@ def gb300_arm(args, rank: int, world: int):
     recs = rs.api.profile_collect()
     for (out, buf, scr) in bufs:
         assert rs.scratch_status(scr, stream) == 0
+    slots = {nm: planned_slots(scr) for (nm, *_), (_, _, scr) in zip(arrays, bufs)}
 
     # end to end first: large host-side work (the oracle's arrays) makes the next host<->device
     # copies of pinned buffers slow for a while (measured: 12-25 GB/s against 190-210 GB/s)
@@ -269,40 +282,49 @@ def gb300_arm(args, rank: int, world: int):
 
     peak, peak_kind = measured_peak()
     # per-sort and per-kernel breakdown from the launch records (launch order is fixed per step)
-    per_sort = {nm: {"ms": 0.0, "sweep_ms": [], "launches": 0} for nm, *_ in arrays}
+    per_sort = {nm: {"ms": 0.0, "sweep_ms": [], "one_ms": [], "launches": 0} for nm, *_ in arrays}
     ours = [r for r in recs if r["kernel"] != "memset"]
-    # every sort's launches start with its memset; the sorts of a step run in the arrays' order
+    # every sort's launches start with its memset (a sort of one tile is one launch); the sorts of a step run in the
+    # arrays' order
     names = [nm for nm, *_ in arrays]
-    sort_i = -1
+    sort_i, prev = -1, None
     for r in recs:
-        if r["kernel"] == "memset":
+        if r["kernel"] == "memset" or (r["kernel"] == "one" and prev != "memset"):
             sort_i += 1
+        prev = r["kernel"]
         nm = names[max(sort_i, 0) % len(names)]
         per_sort[nm]["ms"] += r["ms"]
         if r["kernel"] != "memset":
             per_sort[nm]["launches"] += 1
         if r["kernel"] == "onesweep":
             per_sort[nm]["sweep_ms"].append((r["pass_"], r["ms"]))
+        if r["kernel"] == "one":
+            per_sort[nm]["one_ms"].append(r["ms"])
     per_dtype = {}
     for (nm, bits, kdt, d, m), a in zip(arrays, act):
         kb = bits.element_size()
         t = per_sort[nm]["ms"] / args.steps
-        ran = len(passes_that_ran(per_sort[nm]["sweep_ms"])) // args.steps   # a prefix sort runs fewer than survive
-        a = min(a, ran) if ran else a
+        ran = len(passes_that_ran(per_sort[nm]["sweep_ms"], slots[nm], args.steps)) // args.steps
+        a = ran or a                # a prefix sort runs fewer than survive; a sort that is one kernel has no launches
         algo = a * 2 * kb * n
         per_dtype[nm] = {"gkeys_s": round(n / (t * 1e-3) / 1e9, 3), "ms": round(t, 4), "active_passes": a,
                          "algorithmic_bytes": algo,
                          "roofline_frac": round(algo / (t * 1e-3) / 1e9 / peak, 4)}
     # dominant kernel: onesweep on the 64-bit keys (the passes that ran)
-    sw = passes_that_ran(per_sort["int64_ascfwdorder"]["sweep_ms"])
-    avg_ms = sum(sw) / len(sw)
+    sw = passes_that_ran(per_sort["int64_ascfwdorder"]["sweep_ms"], slots["int64_ascfwdorder"], args.steps)
+    kernel = f"k_onesweep_pipe<uint64, 512 x 16> (int64 sort, {len(sw) // args.steps} active passes)"
     bytes_launch = 2 * 8 * n
+    if not sw:                      # --log2n of a sort that is one kernel
+        sw = per_sort["int64_ascfwdorder"]["one_ms"]
+        kernel = "k_sort_one<uint64> (int64 sort, every pass)"
+        bytes_launch *= per_dtype["int64_ascfwdorder"]["active_passes"]
+    avg_ms = sum(sw) / len(sw)
     achieved = bytes_launch / (avg_ms * 1e-3) / 1e9
     share = {k: 0.0 for k in ("memset", "histogram", "plan", "onesweep", "settle", "copy")}
     for r in recs:
         share[r["kernel"]] = share.get(r["kernel"], 0.0) + r["ms"]
     tot = sum(share.values())
-    roofline = {"bound": "hbm", "kernel": f"k_onesweep_pipe<uint64, 512 x 16> (int64 sort, {len(sw) // args.steps} active passes)",
+    roofline = {"bound": "hbm", "kernel": kernel,
                 "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "peak_source": f"of {peak_kind}",
                 "traffic": profiled_traffic(), "bytes_per_launch": bytes_launch,
@@ -386,15 +408,16 @@ def uniform_u32(args, rs, dev, stream, peak) -> dict:
     ms = t0.elapsed_time(t1) / args.steps
     sw = [r["ms"] for r in recs if r["kernel"] == "onesweep"]
     hist = [r["ms"] for r in recs if r["kernel"] == "histogram"]
+    sweeps = {} if not sw else {             # (none: --log2n of a sort that is one kernel)
+        "onesweep_avg_ms": round(sum(sw) / len(sw), 4),
+        "onesweep_GBps": round(2 * 4 * n / (sum(sw) / len(sw) * 1e-3) / 1e9, 1),
+        "histogram_ms": round(sum(hist) / len(hist), 4)}
     algo = 4 * 2 * 4 * n
     k = out.to(torch.int64) & 0xFFFFFFFF
     ok = bool((k[:-1] <= k[1:]).all())
     del bits, out, buf, scr
     return {"gkeys_s": round(n / (ms * 1e-3) / 1e9, 3), "ms": round(ms, 4),
-            "roofline_frac": round(algo / (ms * 1e-3) / 1e9 / peak, 4),
-            "onesweep_avg_ms": round(sum(sw) / len(sw), 4),
-            "onesweep_GBps": round(2 * 4 * n / (sum(sw) / len(sw) * 1e-3) / 1e9, 1),
-            "histogram_ms": round(sum(hist) / len(hist), 4), "sorted": ok}
+            "roofline_frac": round(algo / (ms * 1e-3) / 1e9 / peak, 4), **sweeps, "sorted": ok}
 
 
 def float32_abs_reverse(args, rs, arrays, stream) -> dict:
@@ -850,7 +873,8 @@ def config3_records(args, rs, dev, stream, peak) -> dict:
     torch.cuda.synchronize()
     assert rs.scratch_status(scr, stream) == 0
     ms = e0.elapsed_time(e1) / args.steps
-    algo = 8 * 2 * 16 * n                     # 8 digit passes x read + write of key and pointer
+    passes = len(planned_slots(scr))          # digit passes that ran (a prefix of the digits)
+    algo = passes * 2 * 16 * n                # x read + write of key and pointer
     got = (out.cpu().numpy() - base) // 24
     rec_h = np.ascontiguousarray(rec.cpu().numpy())
     del rec, ptrs, out, buf, scr
@@ -862,7 +886,7 @@ def config3_records(args, rs, dev, stream, peak) -> dict:
             - np.uint64(hb)) // np.uint64(24)
     ok = bool(np.array_equal(got, want.astype(np.int64)))
     return {"keys": n, "ms": round(ms, 4), "gkeys_s": round(n / (ms * 1e-3) / 1e9, 3),
-            "algorithmic_bytes": algo, "roofline_frac": round(algo / (ms * 1e-3) / 1e9 / peak, 4),
+            "passes": passes, "algorithmic_bytes": algo, "roofline_frac": round(algo / (ms * 1e-3) / 1e9 / peak, 4),
             "checked": "bit-exact pointer order vs oracle" if ok else "FAILED vs oracle"}
 
 

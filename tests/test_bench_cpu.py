@@ -33,6 +33,43 @@ def test_reference_arm_other_ranks_silent():
     assert r.returncode == 0 and r.stdout.strip() == ""
 
 
+def test_passes_that_ran_are_the_plans():
+    """the launches that moved keys are named by the control block, whatever their times: one that took eight times as
+    long as the others changes nothing, and a record too many or too few is an error"""
+    import torch
+    sys.path.insert(0, ROOT)
+    import bench
+    w = torch.zeros(256, dtype=torch.int32)
+    for slot in (0, 1, 2, 9):
+        w[bench.CTRL_PLAN + bench.PLAN_WORDS * slot + bench.PLAN_ACTIVE] = 1
+    slots = bench.planned_slots(w.view(torch.uint8))
+    assert slots == {0, 1, 2, 9}
+    times = [(p, 100.0 if (step, p) == (1, 1) else 1.0 if p in slots else 0.01) for step in range(3) for p in range(14)]
+    assert sorted(bench.passes_that_ran(times, slots, 3)) == [1.0] * 11 + [100.0]
+    with pytest.raises(AssertionError):
+        bench.passes_that_ran(times[1:], slots, 3)
+    assert bench.passes_that_ran([], set(), 3) == []
+
+
+def test_control_block_words_of_the_bench(tmp_path):
+    """the words that bench.py reads are where the library's Control has them"""
+    import shutil
+    sys.path.insert(0, ROOT)
+    import bench
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    src = tmp_path / "ctrl.cu"
+    src.write_text('#include <cstddef>\n#include <cstdio>\n#include "rsbd8g_device.cuh"\nint main() { using namespace rsbd8g; '
+                   'std::printf("%zu %zu %zu %d", offsetof(Control, plan), sizeof(PassPlan), offsetof(PassPlan, active), kMaxSlots); }')
+    exe = str(tmp_path / "ctrl")
+    r = subprocess.run([nvcc, "-std=c++17", "-I", os.path.join(ROOT, "radixsortbidi8_gb300", "csrc"), str(src), "-o", exe],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    got = [int(x) for x in subprocess.run([exe], capture_output=True, text=True).stdout.split()]
+    assert got == [4 * bench.CTRL_PLAN, 4 * bench.PLAN_WORDS, 4 * bench.PLAN_ACTIVE, bench.CTRL_SLOTS]
+
+
 def _worker(rank, world, port, q):
     import torch.distributed as dist
     sys.path.insert(0, ROOT)
