@@ -47,8 +47,8 @@ constexpr uint32_t kSampleRun = 32;
 // pairs, and sort side by side: a bitonic network, by shuffles within a warp and through shared memory
 // beyond.
 // The pairs that the samples can form should outnumber the keys, for one pair too many to show: the smallest
-// size of sample that does (152 samples of 256 keys form 5 M pairs, of 1024 keys 80 M), or several rounds of the
-// largest.  A sample of 1024 keys adds 9 us to the histogram, of 256 keys 4 to 5 (2^21 int64 keys 28.4 -> 24.4 us, 19.1
+// size of sample that does so twice (152 samples of 256 keys form 5 M pairs, of 1024 keys 80 M; with once, 2^24 uniform
+// keys lay so near the line that a fourth pass was taken, 473 us for 440), or several rounds of the largest.  A sample of 1024 keys adds 9 us to the histogram, of 256 keys 4 to 5 (2^21 int64 keys 28.4 -> 24.4 us, 19.1
 // without samples).
 constexpr int kSampleLeast = 256, kSampleDirect = 1024;    // k_histogram: up to one key per thread
 constexpr int kSampleGather = 512;                         // k_gather_histogram: one key per thread (smaller samples took as long)
@@ -56,7 +56,7 @@ __host__ __device__ __forceinline__ uint64_t prefix_pairs(uint32_t samples, uint
 template <int LEAST, int MOST>
 __host__ __device__ __forceinline__ uint32_t prefix_size(uint64_t n, uint32_t samples) {
     uint32_t size = LEAST;
-    while (size < MOST && prefix_pairs(samples, size) < n) size *= 2;
+    while (size < MOST && prefix_pairs(samples, size) < 2 * n) size *= 2;
     return size;
 }
 __host__ __device__ __forceinline__ uint32_t prefix_rounds(uint64_t n, uint32_t samples, uint32_t size) {
@@ -276,9 +276,9 @@ __device__ __forceinline__ void plan_copy(Control *__restrict__ ctrl, const Plan
 // keys keep their order): a round per key that another has to pass, a few for groups of a few keys.
 //   A group that is still open at the end of the halo, or takes more than kRounds rounds, is settled by
 // the warp in shared memory, with kView keys in view, every key moving to the place found by comparing
-// it with its group (settle_wide).  One that runs past the view is settled by the first warp that meets an inversion
-// in it, whichever chunk that is in, after its chunks: by digit passes of its own over the digits below the prefix,
-// through the array that the scatter passes left free (settle_long).
+// it with its group (settle_wide).  One of more than kMost keys, or that runs past the view, is settled by the first
+// warp that meets an inversion in it, whichever chunk that is in, after its chunks: by digit passes of its own over
+// the digits below the prefix, through the array that the scatter passes left free (settle_long).
 //   A group from an earlier chunk is otherwise left alone, as that chunk's warp settles it.  No inversion is passed
 // over: each lies in some warp's chunk, and its group either ends within the view of the chunk it starts in
 // or is taken by settle_long, which raises settle_fail where the group is too long.  Neighbouring chunks read keys
@@ -293,6 +293,7 @@ struct SettleShape {
     static constexpr int kView = kChunk + 224;
     static constexpr int kWords = (kView + 31) / 32;
     static constexpr int kRounds = 12;
+    static constexpr int kMost = 96;        // keys of the longest group that settle_wide settles (its work grows with the square)
 };
 
 // The longest group of n keys that a warp settles: 2 sqrt(n) keys, rounded up.  A crowd of g keys among
@@ -412,18 +413,15 @@ __device__ __forceinline__ int settle_take(const SettleLong<U> &w, unsigned long
     return -1;
 }
 
-// keep an inversion in a long group for settle_long (of the lanes that call it at once, the first one's)
+// keep an inversion in a long group for settle_long (any lanes may call it)
 template <typename U>
 __device__ __noinline__ void settle_later(SettleWarp<U> *warp, uint64_t at, uint32_t *fail, uint32_t fail_bit) {
-    if ((threadIdx.x & 31u) != uint32_t(__ffs(__activemask()) - 1)) return;
-    const uint32_t i = warp->found;
-    if (i < kSettleLater) {
-        warp->later[i] = warp->tag + at;
-        warp->found = i + 1;
-    } else {
-        atomicOr(fail, fail_bit);
-    }
+    const uint32_t i = atomicAdd(&warp->found, 1u);
+    if (i < kSettleLater) warp->later[i] = warp->tag + at;
+    else atomicOr(fail, fail_bit);
 }
+template <typename U>
+__device__ __forceinline__ uint32_t settle_found(const SettleWarp<U> &warp) { return min(warp.found, kSettleLater); }
 
 // the largest d <= most with ok(d), by a warp: 32 probes a round; ok(lo) holds, and ok is true up to that d
 template <typename F>
@@ -473,7 +471,7 @@ __device__ __noinline__ void settle_long(U *keys, uint64_t *vals, uint64_t at, u
     const uint32_t on = warp_last(0, uint32_t(n - 1 - at < limit ? n - 1 - at : limit), [&](uint32_t d) { return same(at + d); });
     const uint32_t len = back + on + 1;
     const uint64_t s = at - back, c0 = s / S::kChunk * S::kChunk;
-    if (s + len < c0 + S::kView || c0 + S::kView >= n) return;      // settle_wide's
+    if (len <= uint32_t(S::kMost) && (s + len < c0 + S::kView || c0 + S::kView >= n)) return;      // settle_wide's
     int mine = -1;
     if (lane == 0 && len <= limit) mine = settle_take(w, s + w.tag + 1u);
     mine = __shfl_sync(0xFFFFFFFFu, mine, 0);
@@ -572,7 +570,10 @@ __device__ __noinline__ void settle_long(U *keys, uint64_t *vals, uint64_t at, u
     __syncwarp();                                         // the warp's shared memory is free again
 }
 
-// one warp settles the groups that start in the chunk at c0, in shared memory
+// One warp settles the groups that start in the chunk at c0, in shared memory: every key of a group that is out of
+// order finds its place by comparing itself with its group, all groups side by side (one group after another took 13 us
+// a chunk of groups of six).  Long ones, and one that runs on past the view, are kept for settle_long (2^23 keys of 64 k
+// values, some of whose groups have 256 keys: 248 us with all of them settled here, 59 so).
 template <int MODE, bool HAS_VAL, typename S, typename U>
 __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, uint64_t n, U mask, bool desc, SettleWarp<U> *warp,
                                          uint32_t *fail, uint32_t fail_bit) {
@@ -598,38 +599,56 @@ __device__ __noinline__ void settle_wide(U *keys, uint64_t *vals, uint64_t c0, u
         }
     }
     __syncwarp();
-    int s = bit_at_or_above(hw, 0, WORDS);                // the first group that starts here
-    while (s < S::kChunk && s < view) {
-        const int x = bit_at_or_above(vw, s, WORDS);      // the next inversion, and its group
-        if (x >= view) break;
-        s = bit_at_or_below(hw, x);
-        if (s >= S::kChunk) break;
-        int e = bit_at_or_above(hw, x + 1, WORDS);
-        if (e >= view) {
-            if (c0 + uint64_t(view) < n) {                // it runs on past the view
-                if (lane == 0) settle_later(warp, c0 + uint64_t(x), fail, fail_bit);
-                break;
-            }
-            e = view;
+    int to[WORDS];                                        // where this lane's keys go (-1: they stay)
+    uint64_t p[HAS_VAL ? WORDS : 1];
+    for (int r = 0; r < WORDS; ++r) {
+        const int i = r * 32 + lane;
+        to[r] = -1;
+        if (i >= view) continue;
+        const int s = bit_at_or_below(hw, i);
+        if (s < 0 || s >= S::kChunk) continue;            // from an earlier chunk, or of the next
+        const int x = bit_at_or_above(vw, s, WORDS), e = bit_at_or_above(hw, i + 1, WORDS);
+        if (x >= e) continue;                             // in order
+        if (e - s > S::kMost || (e == view && c0 + uint64_t(view) < n)) {
+            if (i == x) settle_later(warp, c0 + uint64_t(x), fail, fail_bit);
+            continue;
         }
-        uint64_t p[HAS_VAL ? WORDS : 1];
-        if constexpr (HAS_VAL) {                          // every pointer of the group is read before any is moved
-            for (int i = s + lane, r = 0; i < e; i += 32, ++r) p[r] = vals[c0 + i];
-            __syncwarp();
+        const U b = settle_order<MODE>(key[i], desc);
+        int at = s;
+#pragma unroll 4
+        for (int j = s; j < e; ++j) {
+            const U a = settle_order<MODE>(key[j], desc);
+            at += key_less(a, b) || (j < i && key_same(a, b)) ? 1 : 0;
         }
-        for (int i = s + lane, r = 0; i < e; i += 32, ++r) {
-            const U b = settle_order<MODE>(key[i], desc);
-            int at = s;
-            for (int j = s; j < e; ++j) {
-                const U a = settle_order<MODE>(key[j], desc);
-                at += key_less(a, b) || (j < i && key_same(a, b)) ? 1 : 0;
-            }
-            settle_st<MODE>(keys + c0 + at, key[i]);
-            if constexpr (HAS_VAL) vals[c0 + at] = p[r];
-        }
-        s = e;
+        if (at == i) continue;
+        to[r] = at;
+        if constexpr (HAS_VAL) p[r] = vals[c0 + i];
+    }
+    __syncwarp();                                         // every pointer that moves has been read
+    for (int r = 0; r < WORDS; ++r) {
+        if (to[r] < 0) continue;
+        settle_st<MODE>(keys + c0 + to[r], key[r * 32 + lane]);
+        if constexpr (HAS_VAL) vals[c0 + to[r]] = p[r];
     }
     __syncwarp();                                         // the warp's shared memory is free again
+}
+
+// Does the group of the key at c0 + 255 have an inversion between there and the end of the view?  (Most groups that are
+// open at the halo's end and in order so far stay so, many copies of one key above all: 2^26 keys of 64 k values 186 us
+// with settle_wide for each such chunk, 141 so.)
+template <int MODE, typename S, typename U>
+__device__ __noinline__ bool settle_peek(const U *keys, uint64_t c0, uint64_t n, U mask, bool desc) {
+    constexpr int SEEN = 32 * S::kItems;
+    const int lane = int(threadIdx.x & 31u), view = int(n - c0 < uint64_t(S::kView) ? n - c0 : uint64_t(S::kView));
+    const U last = settle_order<MODE>(settle_ld<MODE>(keys + c0 + SEEN - 1), desc);
+    bool inv = false;
+#pragma unroll
+    for (int j = 0; j < (S::kView - SEEN + 31) / 32; ++j) {
+        const int x = min(SEEN + j * 32 + lane, view - 1);
+        const U a = settle_order<MODE>(settle_ld<MODE>(keys + c0 + x - 1), desc), b = settle_order<MODE>(settle_ld<MODE>(keys + c0 + x), desc);
+        inv |= same_masked(last, b, mask) && key_less(b, a);
+    }
+    return __any_sync(0xFFFFFFFFu, inv) != 0;
 }
 
 // one warp settles the groups that start in the chunk at c0, and keeps what it meets of long groups for later (a
@@ -700,10 +719,13 @@ __device__ __forceinline__ void settle_chunk(U *keys, uint64_t *vals, uint64_t c
             const U a = settle_order<MODE>(settle_ld<MODE>(keys + c0 - C - 1), desc), b = settle_order<MODE>(settle_ld<MODE>(keys + c0 - 1), desc);
             left |= same_masked(a, b, mask);
         }
-        if (left) settle_later(warp, c0 + uint64_t(lane * ITEMS + 31 - __clz(bad_in)), fail, fail_bit);
+        const uint32_t any = __ballot_sync(0xFFFFFFFFu, left);
+        if (left && lane == __ffs(any) - 1) settle_later(warp, c0 + uint64_t(lane * ITEMS + 31 - __clz(bad_in)), fail, fail_bit);
     }
     const uint32_t pass = ~hb & ~in & ~out & 0xFFu;          // keys that may pass the one before them
+    // (open: with no inversion in the group so far, it is looked at on to the view's end)
     bool wide = open;
+    if (open && !__any_sync(0xFFFFFFFFu, (vb & ~in) != 0)) wide = settle_peek<MODE, S>(keys, c0, n, mask, desc);
     if (!open) {
         uint32_t moved = 0, from[INDEX ? ITEMS : 1];
         if constexpr (INDEX) {
@@ -817,7 +839,8 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
     for (uint64_t c0 = uint64_t(blockIdx.x) * S::kCtaKeys + uint32_t(warp * C); c0 < n; c0 += stride)
         settle_chunk<MODE, HAS_VAL, S>(keys, vals, c0, n, mask, desc != 0, &warps[warp], &ctrl->settle_fail, 1u);
     __syncwarp();
-    if (warps[warp].found && !__any_sync(0xFFFFFFFFu, ld_relaxed(&ctrl->settle_fail) != 0)) {
+    const uint32_t found = settle_found(warps[warp]);
+    if (found && !__any_sync(0xFFFFFFFFu, ld_relaxed(&ctrl->settle_fail) != 0)) {
         // the array that is free: what the last pass read from or could have, the copy forms' buffer or the in-place
         // forms' other array; the table of long groups lies where the last digit's look-back words do, which are
         // clear (a prefix leaves two digits out)
@@ -833,7 +856,7 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, sizeof(U) == 8 ? (HA
         w.room = uint32_t(status_bytes / 8 < kTakenRoom ? status_bytes / 8 : kTakenRoom);
         w.digits = survive & ((1u << low) - 1u);
         bad = __any_sync(0xFFFFFFFFu, bad);
-        for (uint32_t i = 0; i < warps[warp].found && !bad; ++i)
+        for (uint32_t i = 0; i < found && !bad; ++i)
             settle_long<MODE, HAS_VAL>(keys, vals, warps[warp].later[i], n, mask, desc != 0, &warps[warp], w, &ctrl->settle_fail, 1u);
     }
     __threadfence();

@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(SettleShape<U>::kThreads, 4) k_seg_settle(SegA
         if (lane == 0 && (ld_relaxed(a.seg_mask + idx) & kSegFail)) atomicOr(&c->pass_mask[1], how & 0xFFFFu);
     }
     __syncwarp();
-    for (uint32_t i = 0; i < warps[warp].found; ++i) {
+    for (uint32_t i = 0, found = settle_found(warps[warp]); i < found; ++i) {
         const uint32_t idx = uint32_t(warps[warp].later[i] >> 32), seg = a.large_seg[idx];
         const uint32_t how = __shfl_sync(0xFFFFFFFFu, ld_relaxed(a.seg_mask + idx), 0);
         if (how & kSegFail) continue;
