@@ -33,30 +33,23 @@ __host__ __device__ __forceinline__ bool a_before_b(U a, U b, bool desc, bool a_
 // warp (all 32 lanes call it with the same arguments): each round probes 32 points of the interval
 // holding the answer and keeps the gap between the last true and the first false probe, so a
 // search over n elements takes about log32(n) dependent loads instead of log2(n)
-// (`at_a(i)` / `at_b(j)`: element i of A, element j of B -- global arrays or the circular windows)
-template <int MODE, typename U, typename I, typename FA, typename FB>
-__device__ __forceinline__ I merge_path_warp_by(FA at_a, I na, FB at_b, I nb, I d, bool desc, bool a_first) {
-    I lo = d > nb ? d - nb : 0, hi = d < na ? d : na;             // the answer lies in [lo, hi]
-    const uint32_t lane = threadIdx.x & 31u;
-    while (hi - lo > 32) {
-        const I p = lo + I(uint64_t(hi - lo) * (lane + 1) / 33);   // 32 increasing points of (lo, hi)
-        const bool t = a_before_b<MODE>(at_a(p), at_b(d - 1 - p), desc, a_first);
-        const int k = __popc(__ballot_sync(0xFFFFFFFFu, t));     // the true probes are a prefix
-        const I below = __shfl_sync(0xFFFFFFFFu, p, k > 0 ? k - 1 : 0);
-        const I above = __shfl_sync(0xFFFFFFFFu, p, k < 32 ? k : 31);
-        if (k > 0) lo = below + 1;
-        if (k < 32) hi = above;
-    }
-    const I p = lo + lane;
-    const bool t = p < hi && a_before_b<MODE>(at_a(p), at_b(d - 1 - p), desc, a_first);
-    return lo + I(__popc(__ballot_sync(0xFFFFFFFFu, t)));
-}
-
 template <int MODE, typename U>
 __device__ __forceinline__ uint64_t merge_path_warp(const U *A, uint64_t na, const U *B, uint64_t nb, uint64_t d,
                                                     bool desc, bool a_first) {
-    return merge_path_warp_by<MODE, U, uint64_t>([A](uint64_t i) { return A[i]; }, na,
-                                                 [B](uint64_t j) { return B[j]; }, nb, d, desc, a_first);
+    uint64_t lo = d > nb ? d - nb : 0, hi = d < na ? d : na;      // the answer lies in [lo, hi]
+    const uint32_t lane = threadIdx.x & 31u;
+    while (hi - lo > 32) {
+        const uint64_t p = lo + (hi - lo) * (lane + 1) / 33;      // 32 increasing points of (lo, hi)
+        const bool t = a_before_b<MODE>(A[p], B[d - 1 - p], desc, a_first);
+        const int k = __popc(__ballot_sync(0xFFFFFFFFu, t));     // the true probes are a prefix
+        const uint64_t below = __shfl_sync(0xFFFFFFFFu, p, k > 0 ? k - 1 : 0);
+        const uint64_t above = __shfl_sync(0xFFFFFFFFu, p, k < 32 ? k : 31);
+        if (k > 0) lo = below + 1;
+        if (k < 32) hi = above;
+    }
+    const uint64_t p = lo + lane;
+    const bool t = p < hi && a_before_b<MODE>(A[p], B[d - 1 - p], desc, a_first);
+    return lo + uint64_t(__popc(__ballot_sync(0xFFFFFFFFu, t)));
 }
 
 // Tiles of kTile outputs, THREADS x kItems: an odd number of outputs per thread, so that the threads'
