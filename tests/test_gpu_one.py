@@ -136,3 +136,26 @@ def test_small_sorts_by_a_launch_per_digit(dtype, mode, direction, n):
     out = torch.empty_like(ptr)
     assert rs.radixsortcopy_member(ptr, out, dtype, 8, direction, mode, flags=api.FLAG_DIAG_LAUNCHES)
     assert np.array_equal((out.cpu().numpy() - dev.data_ptr()) // 24, O.numpy_sort_indices(key, mode, direction))
+
+
+def test_one_kernel_sorts_on_several_streams():
+    """sorts that each want most of the SMs at once, queued on eight streams beside larger and smaller ones"""
+    import torch
+    import radixsortbidi8_gb300 as rs
+    sizes = [1 << 20, 152 * 4096, 152 * 8192, 100003, 1000, (1 << 22) + 3, 1 << 20, 600011]
+    arrs = [S.uniform_bits(i, n, np.uint32) for i, n in enumerate(sizes)]
+    st = []
+    for a in arrs:
+        x = to_dev(a)
+        st.append((x, [torch.empty_like(x) for _ in range(3)], torch.empty_like(x),
+                   torch.empty(rs.scratch_bytes(np.uint32, a.size), dtype=torch.uint8, device="cuda"), torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    for k in range(3):
+        for x, outs, buf, scratch, s in st:
+            rs.radixsortcopynoalloc(x, outs[k], buf, scratch, key_dtype=np.uint32, stream=s)
+    torch.cuda.synchronize()
+    for a, (x, outs, buf, scratch, s) in zip(arrs, st):
+        assert rs.scratch_status(scratch) == 0
+        want = np.sort(a)
+        for y in outs:
+            assert same_bits(from_dev(y, np.uint32), want)
