@@ -47,8 +47,9 @@ constexpr uint32_t kSampleRun = 32;
 // pairs, and sort side by side: a bitonic network, by shuffles within a warp and through shared memory
 // beyond.
 // The pairs that the samples can form should outnumber the keys, for one pair too many to show: the smallest
-// size of sample that does so twice (152 samples of 256 keys form 5 M pairs, of 1024 keys 80 M; with once, 2^24 uniform
-// keys lay so near the line that a fourth pass was taken, 473 us for 440), or several rounds of the largest.  A sample of 1024 keys adds 9 us to the histogram, of 256 keys 4 to 5 (2^21 int64 keys 28.4 -> 24.4 us, 19.1
+// size of sample that forms half as many again (152 samples of 256 keys form 5 M pairs, of 1024 keys 80 M; with no more
+// than the keys, 2^24 uniform ones lay so near the line that a fourth pass was taken, 473 us for 440), or several rounds
+// of the largest.  A sample of 1024 keys adds 9 us to the histogram, of 256 keys 4 to 5 (2^21 int64 keys 28.4 -> 24.4 us, 19.1
 // without samples).
 constexpr int kSampleLeast = 256, kSampleDirect = 1024;    // k_histogram: up to one key per thread
 constexpr int kSampleGather = 512;                         // k_gather_histogram: one key per thread (smaller samples took as long)
@@ -56,7 +57,7 @@ __host__ __device__ __forceinline__ uint64_t prefix_pairs(uint32_t samples, uint
 template <int LEAST, int MOST>
 __host__ __device__ __forceinline__ uint32_t prefix_size(uint64_t n, uint32_t samples) {
     uint32_t size = LEAST;
-    while (size < MOST && prefix_pairs(samples, size) < 2 * n) size *= 2;
+    while (size < MOST && prefix_pairs(samples, size) < n + n / 2) size *= 2;
     return size;
 }
 __host__ __device__ __forceinline__ uint32_t prefix_rounds(uint64_t n, uint32_t samples, uint32_t size) {
