@@ -309,8 +309,7 @@ __host__ __device__ __forceinline__ uint64_t settle_limit(uint64_t n) {
     return m < 1024 ? 1024 : m;
 }
 
-// Inversions in long groups that a warp keeps (more fail the step: crowds are for the samples to see); with 24, the
-// five CTAs of an SM passed 164 KB of shared memory and L1 halved: 2^28 keys 594 -> 624 us.
+// inversions in long groups that a warp keeps (more fail the step: crowds are for the samples to see)
 constexpr uint32_t kSettleLater = 12;
 // a warp's shared memory in the settle step
 template <typename U>
@@ -399,7 +398,6 @@ __device__ __forceinline__ void load_run(U (&v)[ITEMS], const U *p, bool whole) 
     }
 }
 
-
 // take up the long group `id`: 1, or 0 if another warp has, -1 if the table is full
 template <typename U>
 __device__ __forceinline__ int settle_take(const SettleLong<U> &w, unsigned long long id) {
@@ -454,8 +452,8 @@ __device__ __forceinline__ uint32_t diff_digits(uint64_t d) {
 template <int HB>
 __device__ __forceinline__ uint32_t diff_digits(KeyWide<HB> d) { return diff_digits(d.lo) | (diff_digits(d.hi) << 8); }
 
-// One warp sorts the group that has an inversion at key `at`, if it is longer than its chunk's view and no other
-// warp has taken it up: a stable pass per digit below the prefix that is not the same in all, ranked by matching
+// One warp sorts the group that has an inversion at key `at`, unless it is settle_wide's or another warp has taken it
+// up: a stable pass per digit below the prefix that is not the same in all, ranked by matching
 // digits, between the group's place and the same place in the free arrays (a key's place always holds a key of
 // the group, as the neighbours' reads want it).  A pass counts the next one's digits as it goes.
 template <int MODE, bool HAS_VAL, typename U>
